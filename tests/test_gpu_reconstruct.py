@@ -34,6 +34,20 @@ def test_gridding_matches_oracle(shape, post):
         assert np.max(np.abs(g - ref) / np.maximum(np.abs(ref), 1e-6)) < 1e-5
 
 
+@pytest.mark.parametrize("shape", [(1, 3, 5, 257), (2, 1, 3, 601), (3, 7, 1, 33), (1, 1, 1, 1), (2, 5, 17, 65)])
+def test_gridding_row_and_column_remainders(shape):
+    """Row groups that end inside a (b, j, k) carry and column blocks with idle lanes; strided output."""
+    rng = np.random.default_rng(sum(shape))
+    inp = rng.standard_normal(shape).astype(np.float32)
+    ref = np.zeros(shape, dtype=np.float32)
+    assert gridding_correction(inp, ref, post_correction=True) == 0
+    out = torch.full(shape[:3] + (shape[3] + 3,), 7.0, device="cuda")
+    fp.fourier_interpolation_correction(torch.from_numpy(inp).cuda(), out[..., :shape[3]], "linear", True)
+    g = out.cpu().numpy()
+    assert np.max(np.abs(g[..., :shape[3]] - ref) / np.maximum(np.abs(ref), 1e-6)) < 1e-5
+    assert (g[..., shape[3]:] == 7.0).all()
+
+
 def test_gridding_broadcast_constant_and_errors():
     shape = (1, 12, 10, 8)
     out = torch.empty(shape, dtype=torch.float32, device="cuda")
@@ -65,7 +79,7 @@ def _torch_reconstruct(values, weights, n, thr, centered):
     return (real.to(torch.float64) / sinc ** 2)[None]
 
 
-@pytest.mark.parametrize("n,centered", [(32, True), (48, False), (64, True)])
+@pytest.mark.parametrize("n,centered", [(32, True), (48, False), (64, True), (33, True), (130, False)])
 def test_reconstruct_matches_torch_chain(n, centered):
     g = torch.Generator(device="cuda")
     g.manual_seed(n)

@@ -25,7 +25,7 @@ LIB = os.path.join(LIBDIR, "libnoa_b200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
-              "--expt-relaxed-constexpr", "--split-compile=4", "-I", INCLUDE, "-I", CSRC] + ARCH
+              "--expt-relaxed-constexpr", "-I", INCLUDE, "-I", CSRC] + ARCH
 
 
 def nvcc() -> str:

@@ -65,10 +65,15 @@ cudaError_t launch_runs(const ProjArgs& a, const AccGrid& g, cudaStream_t stream
         return cudaSuccess;  // no memory for the accumulator: the caller takes the tile path
     cudaError_t err = cudaMemsetAsync(acc, 0, bytes, stream);
     if (err == cudaSuccess) {
-        const int64_t threads = static_cast<int64_t>(a.slice_w / 2 + 1) * ((a.slice_h + RUN - 1) / RUN);
+        const int64_t wp = a.slice_w / 2 + 1;
+        const int run = run_length(wp, a.slice_h, a.n_slices, sm_count());
+        const int64_t threads = wp * ((a.slice_h + run - 1) / run);
         const dim3 grid(static_cast<unsigned>((threads + RASTER_THREADS - 1) / RASTER_THREADS),
                         static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
-        rasterize_runs_kernel<IN_C, OUT_C, W><<<grid, RASTER_THREADS, 0, stream>>>(a, g, acc);
+        if (run < RUN)
+            rasterize_short_runs_kernel<IN_C, OUT_C, W><<<grid, RASTER_THREADS, 0, stream>>>(a, g, acc, run);
+        else
+            rasterize_runs_kernel<IN_C, OUT_C, W><<<grid, RASTER_THREADS, 0, stream>>>(a, g, acc);
         const int64_t vox = static_cast<int64_t>(a.vol_d) * a.vol_h * (a.vol_w / 2 + 1);
         const int64_t blocks = (vox + 255) / 256;
         const int grid_f = static_cast<int>(blocks < static_cast<int64_t>(sm_count()) * 16 ? blocks : sm_count() * 16);

@@ -78,7 +78,7 @@ rasterize_batch_kernel(const RasterReq* __restrict__ reqs, int n) {
     const int y0 = (t / wp) * RUN;
     if (y0 >= req.a.slice_h)
         return;
-    rasterize_run<IN_C, OUT_C, W>(req.a, req.g, req.acc, b, u, y0);
+    rasterize_run<IN_C, OUT_C, W>(req.a, req.g, req.acc, b, u, y0, RUN);
 }
 
 template<bool OUT_C, bool W>

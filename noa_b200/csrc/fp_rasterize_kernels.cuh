@@ -157,6 +157,18 @@ rasterize_kernel(const __grid_constant__ ProjArgs a, int ntx, void* scratch) {
 // ---------------------------------------------------------------------------------------------------
 constexpr int RUN = 16;
 
+// Rows per thread of a launch: RUN when that gives every SM its four CTAs of threads, else the largest
+// power of two below it that does (down to one row). A run is a serial chain of its rows, so a launch
+// with fewer threads than the chip holds lasts as long as one run: 64 slices of 64^2 as runs of 16 rows
+// are 8,448 threads in 64 half-empty CTAs, 30.7 us a call; as single rows 23.3 us, although the taps that
+// rows share are then reduced one by one.
+inline int run_length(int64_t columns, int64_t rows, int64_t slices, int sms) {
+    int run = RUN;
+    while (run > 1 && columns * ((rows + run - 1) / run) * slices < static_cast<int64_t>(sms) * 1024)
+        run /= 2;
+    return run;
+}
+
 struct AccGrid {
     int r0, r1;     // z and y frequencies held: [-r0, r0], [-r1, r1]
     int n2;         // x frequencies held: [0, n2)
@@ -264,11 +276,11 @@ __device__ __forceinline__ unsigned slide_mask(unsigned m, bool up, bool dn) {
     return m;
 }
 
-// One run: column u, rows [y0, y0 + RUN) of slice b, into the accumulator.
+// One run: column u, rows [y0, y0 + run) of slice b, into the accumulator.
 template<bool IN_C, bool OUT_C, bool W>
 __device__ __forceinline__ void rasterize_run(const ProjArgs& a, const AccGrid& g, void* __restrict__ acc,
-                                              int64_t b, int u, int y0) {
-    const int y_end = min(y0 + RUN, a.slice_h);
+                                              int64_t b, int u, int y0, int run) {
+    const int y_end = min(y0 + run, a.slice_h);
     const bool has_in_w = a.in_w.present;
     const float f1 = div(static_cast<float>(u), a.f_slice1);
     {
@@ -381,7 +393,22 @@ rasterize_runs_kernel(const __grid_constant__ ProjArgs a, const AccGrid g, void*
     if (y0 >= a.slice_h)
         return;
     for (int64_t b = blockIdx.y; b < a.n_slices; b += gridDim.y)
-        rasterize_run<IN_C, OUT_C, W>(a, g, acc, b, u, y0);
+        rasterize_run<IN_C, OUT_C, W>(a, g, acc, b, u, y0, RUN);
+}
+
+// The same with shorter runs (run_length). A kernel of its own: with the run as an argument the kernel
+// above spills more registers and is 5 % slower.
+template<bool IN_C, bool OUT_C, bool W>
+__global__ void __launch_bounds__(RASTER_THREADS, 3)
+rasterize_short_runs_kernel(const __grid_constant__ ProjArgs a, const AccGrid g, void* __restrict__ acc, int run) {
+    const int wp = a.slice_w / 2 + 1;
+    const int t = blockIdx.x * RASTER_THREADS + threadIdx.x;
+    const int u = t % wp;
+    const int y0 = (t / wp) * run;
+    if (y0 >= a.slice_h)
+        return;
+    for (int64_t b = blockIdx.y; b < a.n_slices; b += gridDim.y)
+        rasterize_run<IN_C, OUT_C, W>(a, g, acc, b, u, y0, run);
 }
 
 template<bool OUT_C, bool W>

@@ -22,6 +22,7 @@
 #include "fp_args.cuh"
 #include "fp_pairs.cuh"
 #include "fp_pool.cuh"
+#include "fp_window.cuh"
 #include "noa_b200/batch.h"
 
 #include <algorithm>
@@ -157,6 +158,10 @@ constexpr int N_VARIANTS = 3;
 struct Variant { int ty, tx, wy, wx, min_ctas; };
 constexpr Variant VARIANTS[N_VARIANTS] = {{16, 16, 4, 8, 1}, {8, 32, 2, 16, 1}, {16, 16, 4, 8, 4}};
 
+// Shared memory of one warp of the window kernels; nothing for the others.
+template<int I, bool WINDOW = has_window<I>()> struct BatchSlots { using T = WindowSlots<I>; };
+template<int I> struct BatchSlots<I, false> { struct T {}; };
+
 // PAIRS_ONLY: every request reads a pair copy (LINEAR, complex); the generic path is compiled out so
 // the kernel fits 40 registers (6 CTAs per SM, like extract_pairs_kernel).
 template<int I, bool IN_C, bool OUT_C, int V, bool PAIRS_ONLY = false>
@@ -167,6 +172,7 @@ batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_ite
     constexpr int WORDS = sizeof(BatchReq) / 8;
     __shared__ unsigned long long s_req_words[WORDS];  // the current request, staged once per change
     const BatchReq& R = *reinterpret_cast<const BatchReq*>(s_req_words);
+    __shared__ __align__(16) typename BatchSlots<I>::T s_slots[has_window<I>() ? 8 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int WARPS_X = VT.tx / VT.wx;
     const int ly = (warp / WARPS_X) * VT.wy + lane / VT.wx;
@@ -229,7 +235,12 @@ batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_ite
                 fresh = false;
             }
             const int u = tx * VT.tx + lx;
-            if (u < R.a.slice_w / 2 + 1) {
+            if constexpr (has_window<I>()) {
+                const int y = ty * VT.ty + ly;
+                const bool valid = u < R.a.slice_w / 2 + 1 && y < R.a.slice_h;
+                if (__any_sync(0xffffffffu, valid))
+                    extract_window_patch<I, IN_C, OUT_C, int>(R.a, b, y, u, valid, s_slots[warp], nullptr, 0);
+            } else if (u < R.a.slice_w / 2 + 1) {
                 bool done = false;
                 if constexpr (I == I_LINEAR && IN_C) {
                     if (PAIRS_ONLY || R.pairs) {
@@ -237,7 +248,7 @@ batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_ite
                         done = true;
                     }
                 }
-                if constexpr (!PAIRS_ONLY) {
+                if constexpr (!PAIRS_ONLY && !has_window<I>()) {
                     const int y = ty * VT.ty + ly;
                     if (!done && y < R.a.slice_h)
                         extract_one<I, IN_C, OUT_C>(R.a, b, y, u);

@@ -15,6 +15,9 @@
 #include "fp_args.cuh"
 #include "fp_pairs.cuh"
 #include "fp_pool.cuh"
+#include "fp_window.cuh"
+
+#include <climits>
 
 namespace nb {
 namespace {
@@ -114,8 +117,11 @@ extract_pairs_kernel(const __grid_constant__ ProjArgs a, const float4* __restric
 }
 
 // The w-windowed form over the pair copy: per pixel, the windowed sum over the w offsets of the
-// z-shifted samples, each read as 4 pair loads — extract_kernel's w loop step for step (same offsets,
-// cutoff tests, window values and sum order), so the results are bit-identical to it.
+// z-shifted samples — extract_kernel's w loop step for step (same offsets, cutoff tests, window values
+// and sum order), so the results are bit-identical to it. The offsets are whole z samples, so one
+// sample's cell and the next one's share a z plane: its sum over y and x (the inner part of the sample's
+// sum, in its order) is kept, and each sample but the first reads two pair rows instead of four.
+// 1000 slices of 256^2 with 7 offsets and weights: 1417 us -> 1192 us.
 template<bool OUT_C>
 __global__ void __launch_bounds__(EXTRACT_THREADS)
 extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx) {
@@ -130,6 +136,7 @@ extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restr
     const Spectrum3 sp{a.vol_d, a.vol_h, a.vol_w, a.in_centered};
     const int WP = a.vol_w / 2 + 1;
     const int sz = a.vol_h * WP, sy = WP;
+    const int lo0 = -sp.n0 / 2, hi0 = (sp.n0 - 1) / 2;
     const bool has_out_w = a.out_w.present;
     const float f1 = div(static_cast<float>(u), a.f_slice1);
 
@@ -142,6 +149,13 @@ extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restr
             const float f0 = div(static_cast<float>(index2frequency(a.out_centered, y, a.slice_h)), a.f_slice0);
             float fz, fy, fx;
             slice2grid(f0, f1, a.scale, a.rot, b, a.ews, fz, fy, fx);
+            // What the samples share: the Friedel flip, the y and x cell and its weights.
+            const float qx = mul(fx, a.target2);
+            const bool flip = qx < 0.f;
+            const PairPlane plane(pairs, sz, sy, sp, flip ? -mul(fy, a.target1) : mul(fy, a.target1), flip ? -qx : qx);
+            const int step = flip ? -1 : 1;  // how the z cell moves with w
+            int last_cell = INT_MIN / 2;
+            float2 last = make_float2(0.f, 0.f);
             float2 value = make_float2(0.f, 0.f);
             float weight = 0.f;
             for (int w = 0; w < a.wsize; ++w) {
@@ -150,8 +164,22 @@ extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restr
                 if (dot3(gz, fy, fx, gz, fy, fx) > a.cutoff_sqd)
                     continue;
                 const float cw = w_value(a, s_w, w, off);
-                const float2 iv = to_output<true, OUT_C>(interp_linear_pairs(
-                    pairs, sz, sy, sp, mul(gz, a.target0), mul(fy, a.target1), mul(fx, a.target2)));
+                const float qz = flip ? -mul(gz, a.target0) : mul(gz, a.target0);
+                const float fl = floorf(qz);
+                const int cell = static_cast<int>(fl);
+                const float t = sub(qz, fl);
+                // The plane the cell shares with the previous one, unless rounding moved it otherwise.
+                const int shared = flip ? cell + 1 : cell, fresh = flip ? cell : cell + 1;
+                if (cell - last_cell != step)
+                    last = shared >= lo0 && shared <= hi0 ? plane.sum(shared) : make_float2(0.f, 0.f);
+                const float2 next = fresh >= lo0 && fresh <= hi0 ? plane.sum(fresh) : make_float2(0.f, 0.f);
+                float2 sample = cfma(flip ? next : last, sub(1.f, t), make_float2(0.f, 0.f));
+                sample = cfma(flip ? last : next, t, sample);
+                if (flip)
+                    sample.y = -sample.y;
+                last = next;
+                last_cell = cell;
+                const float2 iv = to_output<true, OUT_C>(sample);
                 value = cadd(value, cmul(iv, cw));
                 if (has_out_w)
                     weight = add(weight, mul(1.f, cw));
@@ -243,6 +271,23 @@ extract_kernel(const __grid_constant__ ProjArgs a, int ntx) {
     }
 }
 
+// Windows of 4 taps and more (fp_window.cuh): each warp owns a 4x8 patch, as in extract_kernel.
+template<int I, bool IN_C, bool OUT_C, typename Idx>
+__global__ void __launch_bounds__(EXTRACT_THREADS, 3)
+extract_window_kernel(const __grid_constant__ ProjArgs a, int ntx) {
+    __shared__ __align__(16) WindowSlots<I> s_slots[EXTRACT_THREADS / 32];
+    __shared__ float s_w[W_TABLE];
+    fill_w_table(a, s_w);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int y = (blockIdx.x / ntx) * TY + (warp >> 1) * 4 + (lane >> 3);
+    const int u = (blockIdx.x % ntx) * TX + (warp & 1) * 8 + (lane & 7);
+    const bool valid = u < a.slice_w / 2 + 1 && y < a.slice_h;
+    if (!__any_sync(0xffffffffu, valid))
+        return;
+    for (int64_t b = blockIdx.y; b < a.n_slices; b += gridDim.y)
+        extract_window_patch<I, IN_C, OUT_C, Idx>(a, b, y, u, valid, s_slots[warp], s_w, W_TABLE);
+}
+
 template<int I, bool IN_C, bool OUT_C>
 cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
     const int wp = a.slice_w / 2 + 1;
@@ -250,10 +295,17 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
     if (a.n_slices == 0)
         return cudaSuccess;
     const dim3 grid(static_cast<unsigned>(ntx * nty), static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
-    if (a.wide_in)
-        extract_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
-    else
-        extract_kernel<I, IN_C, OUT_C, int32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+    if constexpr (has_window<I>()) {
+        if (a.wide_in)
+            extract_window_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+        else
+            extract_window_kernel<I, IN_C, OUT_C, int32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+    } else {
+        if (a.wide_in)
+            extract_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+        else
+            extract_kernel<I, IN_C, OUT_C, int32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+    }
     return cudaGetLastError();
 }
 

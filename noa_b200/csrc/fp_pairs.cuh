@@ -81,6 +81,50 @@ __device__ __forceinline__ float2 interp_linear_pairs(const float4* __restrict__
     return value;
 }
 
+// The y and x part of interp_linear_pairs, for samples that share it: sum(iz) is the sum over the cell's
+// y and x taps in the z plane iz (which lies inside the volume), in interp_linear_pairs' order. `q1` and
+// `q2` are the coordinates after the Friedel flip (q2 >= 0).
+struct PairPlane {
+    const float4* pairs;
+    const Spectrum3 sp;
+    int sz, row0, row1;       // element offsets of the two y rows, at the x cell
+    bool ok0, ok1, okx1;
+    float w10, w11, w20, w21;
+
+    __device__ __forceinline__ PairPlane(const float4* p, int stride_z, int stride_y, const Spectrum3& s, float q1, float q2)
+        : pairs(p), sp(s), sz(stride_z) {
+        const float fl1 = floorf(q1), fl2 = floorf(q2);
+        const int b1 = static_cast<int>(fl1), b2 = static_cast<int>(fl2);
+        w11 = sub(q1, fl1);
+        w21 = sub(q2, fl2);
+        w10 = sub(1.f, w11);
+        w20 = sub(1.f, w21);
+        const int lo1 = -sp.n1 / 2, hi1 = (sp.n1 - 1) / 2, hi2 = sp.n2 / 2;
+        const bool okx0 = b2 >= 0 && b2 <= hi2;
+        ok0 = okx0 && b1 >= lo1 && b1 <= hi1;
+        ok1 = okx0 && b1 + 1 >= lo1 && b1 + 1 <= hi1;
+        okx1 = b2 + 1 <= hi2;
+        row0 = frequency2index(sp.centered, b1, sp.n1) * stride_y + b2;
+        row1 = frequency2index(sp.centered, b1 + 1, sp.n1) * stride_y + b2;
+    }
+
+    __device__ __forceinline__ float2 row(const float4 p) const {
+        float2 v = cfma(make_float2(p.x, p.y), w20, make_float2(0.f, 0.f));
+        return okx1 ? cfma(make_float2(p.z, p.w), w21, v) : v;
+    }
+
+    __device__ __forceinline__ float2 sum(int iz) const {
+        const int oz = frequency2index(sp.centered, iz, sp.n0) * sz;
+        float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
+        if (ok0)
+            p0 = ldg_evict_last_half(pairs + (oz + row0));
+        if (ok1)
+            p1 = ldg_evict_last_half(pairs + (oz + row1));
+        const float2 v = cfma(row(p0), w10, make_float2(0.f, 0.f));
+        return cfma(row(p1), w11, v);
+    }
+};
+
 // slice2grid for a Mat33 rotation with no scaling and no Ewald curvature, when the slice's matrix
 // column 0 is finite: rotate() computes ((m_k0 * 0) + (m_k1 * f0)) + (m_k2 * f1), and for finite m_k0
 // the first product is a zero whose sign never reaches the result (the coordinates then decide the

@@ -1,0 +1,49 @@
+"""GPU kernels at the edges of their tiles and dispatch rules, against the oracle (relative L2 1e-5, the
+tolerance of the same call in test_gpu_parity.py; 1e-4 for the rasterizer's atomic sums)."""
+import numpy as np
+import pytest
+
+from cases import build, clone, default_case, rel_l2
+from oracle.oracle import FpOracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(case, tol, **kw):
+    import gpu_run
+    call = build(case)
+    ref = clone(call)
+    assert FpOracle().run(ref, 8) == 0
+    out, out_w = gpu_run.run(clone(call), **kw)
+    assert rel_l2(out, ref.out) <= tol
+    if ref.out_w is not None:
+        assert rel_l2(out_w, ref.out_w) <= tol
+
+
+# Warp patches of 4x8 pixels that the slice fills partly, cells across x = 0 and the edges of the volume
+# (cutoff beyond 0.5), every window size, both value kinds, input weights, the w-window.
+@pytest.mark.parametrize("interp", ["cubic", "cubic_bspline", "lanczos4", "lanczos6", "lanczos8"])
+@pytest.mark.parametrize("kw", [
+    dict(n=9, slice_n=9, remap="h2h", cutoff=0.8),
+    dict(n=33, slice_n=21, remap="hc2hc", in_w=True, out_w=True),
+    dict(n=26, slice_n=17, remap="h2hc", in_dt="f32", out_dt="f32", cutoff=0.7, out_w=True),
+    dict(n=24, remap="hc2h", w_sinc=(0.05, 0.12), out_w=True, in_w=True),
+], ids=["tiny", "weights", "real", "w-window"])
+def test_window_extraction(interp, kw):
+    _check(default_case("extract", interp=interp, nslices=3, seed=701, **kw), 1e-5)
+
+
+# Run lengths of 1, 2, 4, 8 and 16 rows (148 SMs x 1024 threads decide), the last run of a column shorter.
+@pytest.mark.parametrize("nslices", [7, 400, 800, 1600, 3200])
+def test_rasterize_run_lengths(nslices):
+    _check(default_case("rasterize", n=40, nslices=nslices, remap="h2hc", out_w=True, seed=702), 1e-4)
+
+
+# The planes that a pixel's z samples share: more samples than planes of the volume, offsets outside it, a
+# window wider than the table, odd sizes, power spectra.
+@pytest.mark.parametrize("kw", [dict(n=16, w_sinc=(0.05, 0.9), cutoff=0.9), dict(n=17, w_sinc=(-1.0, 0.2), remap="h2h"),
+                                dict(n=64, nslices=160, w_sinc=(0.1, 0.6), cutoff=0.7),
+                                dict(n=20, w_sinc=(-1.0, 0.15), out_dt="f32")],
+                         ids=["beyond", "odd", "long", "power"])
+def test_w_window_planes(kw):
+    _check(default_case("extract", **{"nslices": 48, "remap": "hc2h", "out_w": True, "seed": 703, **kw}), 1e-5)

@@ -81,6 +81,12 @@ int finish_launch(cudaError_t err);
 // Sets the thread's last error and returns `code`.
 int report_error(int code, const char* message);
 
+// Offset `w` of the w-windowed extraction: (its shift along z, the window's value there).
+__device__ __forceinline__ float2 w_sample(const ProjArgs& a, int w) {
+    const float off = div(static_cast<float>(w - a.wsize / 2), a.target0);
+    return make_float2(off, windowed_sinc(off, a.efs, a.efb));
+}
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

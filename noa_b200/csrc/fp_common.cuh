@@ -293,6 +293,38 @@ __device__ __forceinline__ float2 cfma(float2 a, float s, float2 acc) {
     return make_float2(fmaf(s, a.x, acc.x), fmaf(s, a.y, acc.y));
 }
 
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// Two single-precision fused multiply-adds, each rounded as fmaf, in one instruction.
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The trilinear sum of a 2x2x2 cell of complex values, e[4 z + 2 y + x], in the order of
+// interp_linear_3d: over x, then y, then z.
+__device__ __forceinline__ float2 trilinear(const unsigned long long (&e)[8], float t0, float t1, float t2) {
+    const unsigned long long x0 = pack2(sub(1.f, t2), sub(1.f, t2)), x1 = pack2(t2, t2);
+    const unsigned long long y0 = pack2(sub(1.f, t1), sub(1.f, t1)), y1 = pack2(t1, t1);
+    unsigned long long v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        v[k] = fma2(e[2 * k + 1], x1, fma2(e[2 * k], x0, 0ull));
+    const unsigned long long a = fma2(v[1], y1, fma2(v[0], y0, 0ull)), b = fma2(v[3], y1, fma2(v[2], y0, 0ull));
+    return unpack2(fma2(b, pack2(t0, t0), fma2(a, pack2(sub(1.f, t0), sub(1.f, t0)), 0ull)));
+}
+
 // Spectrum geometry of one rfft input: logical sizes (last one is the full width) and centering.
 struct Spectrum3 { int n0, n1, n2; bool centered; };
 struct Spectrum2 { int n0, n1; bool centered; bool narrow = false; };  // narrow: in-slice offsets fit 32 bits
@@ -478,6 +510,15 @@ struct View3 {
     Idx s0, s1, s2;
 };
 
+// Whether every tap of the trilinear cell at frequencies (b0, b1, b2), b2 >= 0, lies in the spectrum and
+// its rows are adjacent in memory (not across the non-centered layout's wrap at -1).
+__device__ __forceinline__ bool interior_cell(const Spectrum3& sp, int b0, int b1, int b2) {
+    return static_cast<unsigned>(b0 + sp.n0 / 2) < static_cast<unsigned>(sp.n0 - 1) &&
+           static_cast<unsigned>(b1 + sp.n1 / 2) < static_cast<unsigned>(sp.n1 - 1) &&
+           static_cast<unsigned>(b2) < static_cast<unsigned>(sp.n2 / 2) &&
+           (sp.centered || (b0 != -1 && b1 != -1));
+}
+
 // Read-only 16-byte load whose line is kept in L2 with evict_last priority for half of the lines.
 // Volumes (and their pair copies) are about the size of the L2 or larger while the output slices
 // stream past them; keeping part of them resident saves re-reads (bit-identical; 1 % per extraction
@@ -491,6 +532,13 @@ __device__ __forceinline__ float4 ldg_evict_last_half(const float4* p) {
     asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
     return v;
+}
+
+// The same, as the two complex values it holds.
+__device__ __forceinline__ void ldg_pair(const float4* p, unsigned long long& e0, unsigned long long& e1) {
+    unsigned long long pol;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(pol));
+    asm volatile("ld.global.nc.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;" : "=l"(e0), "=l"(e1) : "l"(p), "l"(pol));
 }
 
 template<bool CPLX, typename Idx>
@@ -514,6 +562,22 @@ __device__ __forceinline__ float2 interp_linear_3d(const View3<Idx>& v, const Sp
     const float fl0 = floorf(q0), fl1 = floorf(q1), fl2 = floorf(q2);
     const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1), b2 = static_cast<int>(fl2);
     const float t0 = sub(q0, fl0), t1 = sub(q1, fl1), t2 = sub(q2, fl2);
+    // Interior cells: the same terms in the same order from one base offset, all loads issued together.
+    if constexpr (CPLX) {
+        if (interior_cell(sp, b0, b1, b2)) {
+            const float2* p = static_cast<const float2*>(v.data) +
+                              (static_cast<Idx>(frequency2index(sp.centered, b0, sp.n0)) * v.s0 +
+                               static_cast<Idx>(frequency2index(sp.centered, b1, sp.n1)) * v.s1 + static_cast<Idx>(b2) * v.s2);
+            unsigned long long e[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                e[k] = __ldg(reinterpret_cast<const unsigned long long*>(
+                    p + ((k & 4 ? v.s0 : 0) + (k & 2 ? v.s1 : 0) + (k & 1 ? v.s2 : 0))));
+            float2 value = trilinear(e, t0, t1, t2);
+            value.y *= conjugate;
+            return value;
+        }
+    }
     const float w0[2] = {sub(1.f, t0), t0};
     const float w1[2] = {sub(1.f, t1), t1};
     const float w2[2] = {sub(1.f, t2), t2};

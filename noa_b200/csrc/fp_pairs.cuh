@@ -20,6 +20,20 @@ __device__ __forceinline__ float2 interp_linear_pairs(const float4* __restrict__
     const float fl0 = floorf(q0), fl1 = floorf(q1), fl2 = floorf(q2);
     const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1), b2 = static_cast<int>(fl2);
     const float t0 = sub(q0, fl0), t1 = sub(q1, fl1), t2 = sub(q2, fl2);
+    // Interior cells: the same terms in the same order, from one base offset, with the four loads issued
+    // together.
+    if (interior_cell(sp, b0, b1, b2)) {
+        const float4* p = pairs + (frequency2index(sp.centered, b0, sp.n0) * sz +
+                                   frequency2index(sp.centered, b1, sp.n1) * sy + b2);
+        unsigned long long e[8];
+        ldg_pair(p, e[0], e[1]);
+        ldg_pair(p + sy, e[2], e[3]);
+        ldg_pair(p + sz, e[4], e[5]);
+        ldg_pair(p + sz + sy, e[6], e[7]);
+        float2 value = trilinear(e, t0, t1, t2);
+        value.y *= conjugate;
+        return value;
+    }
     const float w0[2] = {sub(1.f, t0), t0};
     const float w1[2] = {sub(1.f, t1), t1};
     const float w20 = sub(1.f, t2);
@@ -29,33 +43,6 @@ __device__ __forceinline__ float2 interp_linear_pairs(const float4* __restrict__
     const bool okx0 = b2 >= 0 && b2 <= hi2;
     const bool okx1 = b2 + 1 >= 0 && b2 + 1 <= hi2;
     float2 value = make_float2(0.f, 0.f);
-    // Interior cells (every tap inside the volume, the two rows of each axis adjacent in memory: not
-    // across the non-centered layout's wrap at -1): the same terms in the same order, from one base
-    // offset, with the four loads issued together.
-    if (b0 >= lo0 && b0 + 1 <= hi0 && b1 >= lo1 && b1 + 1 <= hi1 && okx0 && okx1 &&
-        (sp.centered || (b0 != -1 && b1 != -1))) {
-        const float4* p = pairs + (frequency2index(sp.centered, b0, sp.n0) * sz +
-                                   frequency2index(sp.centered, b1, sp.n1) * sy + b2);
-        float4 q[4];
-        q[0] = ldg_evict_last_half(p);
-        q[1] = ldg_evict_last_half(p + sy);
-        q[2] = ldg_evict_last_half(p + sz);
-        q[3] = ldg_evict_last_half(p + sz + sy);
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-            float2 vz = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-                float2 vy = make_float2(0.f, 0.f);
-                vy = cfma(make_float2(q[z * 2 + y].x, q[z * 2 + y].y), w20, vy);
-                vy = cfma(make_float2(q[z * 2 + y].z, q[z * 2 + y].w), t2, vy);
-                vz = cfma(vy, w1[y], vz);
-            }
-            value = cfma(vz, w0[z], value);
-        }
-        value.y *= conjugate;
-        return value;
-    }
 #pragma unroll
     for (int z = 0; z < 2; ++z) {
         const int iz = b0 + z;

@@ -21,25 +21,6 @@
 
 namespace nb {
 
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
-// Two single-precision fused multiply-adds, each rounded as fmaf, in one instruction.
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 template<int I>
 struct WindowSlots {
     static constexpr int SIZE = InterpTraits<I>::SIZE;
@@ -150,10 +131,10 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
 }
 
 // One pixel (b, y, u) per lane of slice extraction `a`: all lanes of the warp call it together, those
-// without a pixel with valid = false. `table`: the w-window's values (fill_w_table), or null.
+// without a pixel with valid = false. `table`: the first `table_size` w_sample values.
 template<int I, bool IN_C, bool OUT_C, typename Idx>
 __device__ __forceinline__ void extract_window_patch(const ProjArgs& a, int64_t b, int y, int u, bool valid,
-                                                     WindowSlots<I>& s, const float* table, int table_size) {
+                                                     WindowSlots<I>& s, const float2* table, int table_size) {
     using S = WindowSlots<I>;
     const Spectrum3 sp{a.vol_d, a.vol_h, a.vol_w, a.in_centered};
     const View3<Idx> vol{a.in.data, static_cast<Idx>(a.in.s0), static_cast<Idx>(a.in.s1), static_cast<Idx>(a.in.s2)};
@@ -173,9 +154,9 @@ __device__ __forceinline__ void extract_window_patch(const ProjArgs& a, int64_t 
     for (int w = 0; w < steps; ++w) {
         float gz = fz, cw = 1.f;
         if (a.wsize > 1) {
-            const float off = div(static_cast<float>(w - a.wsize / 2), a.target0);
-            gz = add(fz, off);
-            cw = table && w < table_size ? table[w] : windowed_sinc(off, a.efs, a.efb);
+            const float2 offset = w < table_size ? table[w] : w_sample(a, w);
+            gz = add(fz, offset.x);
+            cw = offset.y;
         }
         const float sqd = dot3(gz, fy, fx, gz, fy, fx);
         const bool inside = valid && (a.wsize > 1 ? !(sqd > a.cutoff_sqd) : sqd <= a.cutoff_sqd);

@@ -47,3 +47,14 @@ def test_rasterize_run_lengths(nslices):
                          ids=["beyond", "odd", "long", "power"])
 def test_w_window_planes(kw):
     _check(default_case("extract", **{"nslices": 48, "remap": "hc2h", "out_w": True, "seed": 703, **kw}), 1e-5)
+
+
+# LINEAR extraction: several slices per CTA with a shorter last group, rows past the slice, cells at the
+# edges of the volume and the non-centered wrap, with and without the pair copy.
+@pytest.mark.parametrize("remap", ["h2h", "hc2hc"])
+@pytest.mark.parametrize("kw", [dict(n=20, nslices=1030), dict(n=21, slice_n=70, nslices=513, target=(1, 70, 70, 70), cutoff=0.9),
+                                dict(n=64, nslices=301, in_w=True, out_w=True), dict(n=40, nslices=800, out_dt="f32", out_w=True),
+                                dict(n=40, nslices=800, in_dt="f32", out_dt="f32")],
+                         ids=["pairs", "beyond", "weights", "power", "real"])
+def test_linear_extraction_groups(kw, remap):
+    _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5)

@@ -198,6 +198,22 @@ __device__ __forceinline__ float windowed_sinc(float fftfreq, float fftfreq_sinc
     return mul(sinc, blackman);
 }
 
+// sin(pi |s|), for |s| < 2^22: |s| minus the nearest integer (exact), an odd polynomial on [-1/2, 1/2]
+// (five terms fitted for the smallest relative error, 5.3e-9 before rounding; 2e-7 in single precision),
+// and the sign of the integer's parity.
+__device__ __forceinline__ float sinpi_reduced(float s) {
+    constexpr float ROUND = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer, held in the low bits
+    s = fabsf(s);
+    const float t = add(s, ROUND);
+    const float r = sub(s, sub(t, ROUND));
+    const float u = r * r;
+    float p = fmaf(0.07756046f, u, -0.59824216f);
+    p = fmaf(p, u, 2.5500698f);
+    p = fmaf(p, u, -5.16771f);
+    p = fmaf(p, u, 3.1415927f);
+    return __int_as_float(__float_as_int(r * p) ^ (__float_as_int(t) << 31));
+}
+
 // The same window for the hot loops of the windowed-sinc insertions, where it only scales a term (the
 // |fftfreq| <= fftfreq_blackman decision is taken before, on exactly rounded coordinates, and the window
 // is 0 at that bound, so nothing discontinuous depends on it): the divisions by fftfreq_sinc and
@@ -205,20 +221,16 @@ __device__ __forceinline__ float windowed_sinc(float fftfreq, float fftfreq_sinc
 // division an approximate one, cos(2 b) is 2 cos(b)^2 - 1, and the Blackman cosine, whose argument
 // stays within [-pi, pi], is the hardware approximation __cosf (6-10 % faster insertions). The sinc's
 // sine is not __sinf: its argument reaches several pi, where __sinf's error grew the insertions' error
-// to 1e-4. Relative difference from windowed_sinc: a few 1e-7.
-// SINPI: the sinc's sine as sinpif(fftfreq * (1 / fftfreq_sinc)) rather than sinf(xs): 8.5 % faster in
-// the gather insertion and 5.5 % in insert_and_extract, 11 % slower in the scatter form (each measured
-// in one call), so those two use it; the two forms differ by 2e-7 (relative L2). sinpif's argument is
-// the sinc's phase in units of pi, rounded twice (the reciprocal, then the product), and xs only feeds
-// the division.
-template<bool SINPI = false>
+// to 1e-4. Its phase is taken in units of pi, so that reducing it is exact; the phase is capped where
+// sinc is below 1e-7 (2^21 periods) to stay in sinpi_reduced's range. Relative difference from
+// windowed_sinc: a few 1e-7.
 __device__ __forceinline__ float windowed_sinc_fast(float fftfreq, float pi_over_sinc, float inv_sinc,
                                                     float pi_over_blackman) {
-    const float xs = fftfreq * pi_over_sinc;
-    const float sn = SINPI ? sinpif(fftfreq * inv_sinc) : sinf(xs);
+    const float xs = fabsf(fftfreq) * pi_over_sinc;
+    const float sn = sinpi_reduced(fminf(fabsf(fftfreq) * inv_sinc, 2097152.f));
     const float sinc = xs == 0.f ? 1.f : __fdividef(sn, xs);
     const float c = __cosf(fftfreq * pi_over_blackman);
-    const float blackman = 0.42f + 0.5f * c + 0.08f * (2.f * c * c - 1.f);
+    const float blackman = fmaf(c, fmaf(c, 0.16f, 0.5f), 0.34f);  // 0.42 + 0.5 cos b + 0.08 cos 2b
     return sinc * blackman;
 }
 

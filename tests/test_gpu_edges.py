@@ -49,6 +49,18 @@ def test_w_window_planes(kw):
     _check(default_case("extract", **{"nslices": 48, "remap": "hc2h", "out_w": True, "seed": 703, **kw}), 1e-5)
 
 
+# LINEAR insertion from Mat33 rotations: bricks that the volume fills partly, more slices than one pass of
+# the list, both layouts, value kinds, input weights, windows from one voxel to wider than the volume.
+@pytest.mark.parametrize("scatter", [False], ids=["gather"])
+@pytest.mark.parametrize("kw", [dict(n=9, nslices=300, out_w=True), dict(n=17, nslices=40, sinc=(0.06, 0.4), remap="hc2hc"),
+                                dict(n=20, nslices=30, slice_n=15, in_w=True, out_w=True, remap="h2hc", cutoff=0.8),
+                                dict(n=16, nslices=20, in_dt="f32", out_dt="f32", in_w=True, out_w=True, sinc=(-1.0, 1.5)),
+                                dict(n=24, nslices=270, in_dt="c32", out_dt="f32", remap="h2h", sinc=(-1.0, 0.2))],
+                         ids=["small", "wide", "weights", "real", "power"])
+def test_linear_insertion(kw, scatter):
+    _check(default_case("insert", **{"seed": 704, **kw}), 1e-5, scatter=scatter)
+
+
 # LINEAR extraction: several slices per CTA with a shorter last group, rows past the slice, cells at the
 # edges of the volume and the non-centered wrap, with and without the pair copy.
 @pytest.mark.parametrize("remap", ["h2h", "hc2hc"])

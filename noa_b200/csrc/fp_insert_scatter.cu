@@ -16,8 +16,10 @@
 // allocated: both run the gather form.
 #include "fp_args.cuh"
 #include "fp_pool.cuh"
+#include "fp_slice_taps.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace nb {
 namespace {
@@ -112,6 +114,105 @@ insert_scatter_kernel(const __grid_constant__ ProjArgs a, void* __restrict__ acc
     }
 }
 
+// The LINEAR form for Mat33 rotations without scaling, from slices whose inner offsets fit 32 bits:
+// insert_scatter_kernel's terms for few instructions per (voxel, slice) pair, which is what bounds it:
+// 500 slices into 256^3 with half-width 6 and weights 2620 us -> 1676 us.
+//
+// The axis that the columns run along is a compile-time constant (the slice picks one of three bodies), so
+// the products of the matrix with the column's two fixed frequencies, and the accumulator offset, are
+// computed once per column; the frequencies come from a table per CTA instead of divisions; and the k
+// range is widened by its rounding error instead of a whole voxel each side.
+template<int AX, bool IN_C, bool W>
+__device__ __forceinline__ void scatter_column(const ProjArgs& a, void* acc, const float* freq, int col, int64_t slice,
+                                               const float* m) {
+    constexpr int P = AX == 0 ? 1 : 0, Q = AX == 2 ? 1 : 2;  // the column's fixed axes, Q fastest
+    const int D = a.vol_d, H = a.vol_h, WP = a.vol_w / 2 + 1;
+    const int extent[3] = {D, H, WP}, lo[3] = {-D / 2, -H / 2, 0}, table[3] = {0, D, D + H};
+    const int stride[3] = {H * WP, WP, 1};
+    if (col >= extent[P] * extent[Q])
+        return;
+    const int ip = col / extent[Q], iq = col - ip * extent[Q];
+    const float fp = freq[table[P] + ip], fq = freq[table[Q] + iq];
+    if (fp * fp + fq * fq > a.cutoff_sqd * 1.0001f)
+        return;  // every voxel of the column is outside the cutoff
+    const float* fa = freq + table[AX];
+    const float target = AX == 0 ? a.target0 : AX == 1 ? a.target1 : a.target2;
+    const float slope = m[AX] / target;  // of the distance to the slice, per index
+    int first = 0, last = extent[AX] - 1;
+    if (fabsf(slope) > 1e-30f) {
+        const float s = m[P] * fp + m[Q] * fq;
+        const float t0 = (-a.fb - s) / slope, t1 = (a.fb - s) / slope;
+        // s and the exact test below are each off by a few 1e-7 of the sum of their terms' sizes.
+        const float slack = 0.01f + 4e-6f * (fabsf(m[P] * fp) + fabsf(m[Q] * fq) + a.fb) / fabsf(slope);
+        // clamped in float first: the range stays within the axis whatever t0, t1 are (NaN included)
+        first = static_cast<int>(fmaxf(ceilf(fminf(t0, t1) - slack) - static_cast<float>(lo[AX]), 0.f));
+        last = static_cast<int>(fminf(floorf(fmaxf(t0, t1) + slack) - static_cast<float>(lo[AX]), static_cast<float>(last)));
+    }
+    const Spectrum2 sp{a.slice_h, a.slice_w, a.in_centered, true};
+    const bool vc = a.out_centered, has_in_w = a.in_w.present;
+    const auto index = [vc](int k, int n) { return frequency2index(vc, k, n); };
+    // Offset of the column; x frequencies are their indices.
+    const int offset = index(lo[P] + ip, extent[P]) * stride[P] + (Q == 2 ? iq : index(lo[Q] + iq, extent[Q]) * stride[Q]);
+    const int s1 = static_cast<int>(a.in.s1), s2 = static_cast<int>(a.in.s2);
+    using T = typename std::conditional<IN_C, float2, float>::type;
+    const T* base = static_cast<const T*>(a.in.data) + slice * a.in.s0;
+    const float* base_w = has_in_w ? static_cast<const float*>(a.in_w.data) + slice * a.in_w.s0 : nullptr;
+    // v0 z + v1 y + v2 x summed in that order, the terms of the fixed axes given.
+    const auto dot = [](float run, float p, float q) {
+        return AX == 0 ? add(add(run, p), q) : AX == 1 ? add(add(p, run), q) : add(add(p, q), run);
+    };
+    const float pp = mul(fp, fp), qq = mul(fq, fq);
+    const float p0 = mul(m[P], fp), q0 = mul(m[Q], fq), p1 = mul(m[3 + P], fp), q1 = mul(m[3 + Q], fq);
+    const float p2 = mul(m[6 + P], fp), q2 = mul(m[6 + Q], fq);
+    for (int k = first; k <= last; ++k) {
+        // The gather form's term (fp_insert.cu, FourierProject.hpp:479-518).
+        const float f = fa[k];
+        const float zz = dot(mul(m[AX], f), p0, q0);
+        if (!(fabsf(zz) <= a.fb) || dot(mul(f, f), pp, qq) > a.cutoff_sqd)
+            continue;
+        const float window = windowed_sinc_fast(zz, a.pfs, a.ifs, a.pfb);
+        const LinearCell cell(sp, mul(dot(mul(m[3 + AX], f), p1, q1), a.f_slice0),
+                              mul(dot(mul(m[6 + AX], f), p2, q2), a.f_slice1));
+        const float2 v = cmul(cell.read(base, s1, s2), window);
+        float w = 0.f;
+        if constexpr (W)
+            w = has_in_w ? mul(cell.read(base_w, static_cast<int>(a.in_w.s1), static_cast<int>(a.in_w.s2)).x, window) : window;
+        acc_red<IN_C, W>(acc, offset + (AX == 2 ? k : index(lo[AX] + k, extent[AX]) * stride[AX]), v, w);
+    }
+}
+
+// Frequencies of one CTA's table: all indices of the three axes.
+constexpr int SCATTER_TABLE = 8192;
+
+template<bool IN_C, bool W>
+__global__ void __launch_bounds__(SCATTER_THREADS)
+scatter_linear_kernel(const __grid_constant__ ProjArgs a, void* __restrict__ acc) {
+    extern __shared__ float s_freq[];
+    const int D = a.vol_d, H = a.vol_h, WP = a.vol_w / 2 + 1;
+    for (int i = threadIdx.x; i < D + H + WP; i += SCATTER_THREADS) {
+        const int k = i < D ? i - D / 2 : i < D + H ? i - D - H / 2 : i - D - H;
+        s_freq[i] = div(static_cast<float>(k), i < D ? a.target0 : i < D + H ? a.target1 : a.target2);
+    }
+    __syncthreads();
+    const int col = blockIdx.x * SCATTER_THREADS + threadIdx.x;
+    for (int64_t i = blockIdx.y; i < a.n_slices; i += gridDim.y) {
+        const float* m = xform_ptr(a.rot, i, 12);
+        const float c0 = fabsf(m[0] / a.target0), c1 = fabsf(m[1] / a.target1), c2 = fabsf(m[2] / a.target2);
+        if (c0 >= c1 && c0 >= c2)
+            scatter_column<0, IN_C, W>(a, acc, s_freq, col, i, m);
+        else if (c1 >= c2)
+            scatter_column<1, IN_C, W>(a, acc, s_freq, col, i, m);
+        else
+            scatter_column<2, IN_C, W>(a, acc, s_freq, col, i, m);
+    }
+}
+
+// Whether scatter_linear_kernel applies.
+bool use_linear_scatter(const ProjArgs& a) {
+    return linear_slices(a) && a.rot.kind == 2 && a.scale.kind == 0 &&
+           static_cast<int64_t>(a.vol_d) + a.vol_h + a.vol_w / 2 + 1 <= SCATTER_TABLE;
+}
+
 // Caller's grids += the accumulator (dense, the caller's index order), converted to the output type.
 template<bool IN_C, bool OUT_C, bool W>
 __global__ void scatter_finalize_kernel(const __grid_constant__ ProjArgs a, const void* __restrict__ acc) {
@@ -152,7 +253,12 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream, bool& done) {
         const int64_t cols = std::max(H * WP, std::max(D * WP, D * H));
         const dim3 grid(static_cast<unsigned>((cols + SCATTER_THREADS - 1) / SCATTER_THREADS),
                         static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
-        insert_scatter_kernel<I, IN_C, W><<<grid, SCATTER_THREADS, 0, stream>>>(a, acc);
+        if (I == I_LINEAR && use_linear_scatter(a)) {
+            const size_t table = static_cast<size_t>(D + H + WP) * sizeof(float);
+            scatter_linear_kernel<IN_C, W><<<grid, SCATTER_THREADS, table, stream>>>(a, acc);
+        } else {
+            insert_scatter_kernel<I, IN_C, W><<<grid, SCATTER_THREADS, 0, stream>>>(a, acc);
+        }
         const int64_t blocks = (vox + 255) / 256;
         const int grid_f = static_cast<int>(blocks < static_cast<int64_t>(sm_count()) * 16 ? blocks : sm_count() * 16);
         scatter_finalize_kernel<IN_C, OUT_C, W><<<grid_f, 256, 0, stream>>>(a, acc);

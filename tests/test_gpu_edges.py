@@ -51,7 +51,7 @@ def test_w_window_planes(kw):
 
 # LINEAR insertion from Mat33 rotations: bricks that the volume fills partly, more slices than one pass of
 # the list, both layouts, value kinds, input weights, windows from one voxel to wider than the volume.
-@pytest.mark.parametrize("scatter", [False], ids=["gather"])
+@pytest.mark.parametrize("scatter", [False, True], ids=["gather", "scatter"])
 @pytest.mark.parametrize("kw", [dict(n=9, nslices=300, out_w=True), dict(n=17, nslices=40, sinc=(0.06, 0.4), remap="hc2hc"),
                                 dict(n=20, nslices=30, slice_n=15, in_w=True, out_w=True, remap="h2hc", cutoff=0.8),
                                 dict(n=16, nslices=20, in_dt="f32", out_dt="f32", in_w=True, out_w=True, sinc=(-1.0, 1.5)),

@@ -9,11 +9,22 @@
 // compacting its own range of slice indices so that building the list needs no barrier; each warp then
 // re-tests the whole list against its own box (one candidate per lane) and walks the survivors' ballot
 // in lane order, with no barrier until the next pass.
+//
+// A third of the warp's pixels lie within a surviving slice's slab, so the walk only computes the distances
+// to it and queues the (pixel, slice) pairs inside, and the warp evaluates queued pairs 32 at a time, one
+// per lane, whichever pixels they belong to: window and interpolation run with all lanes busy. Each lane
+// keeps the queue slots of its own pixel's pairs as a bit mask and adds their results in slot order.
+// 2000 input to 64 output slices of 256^2, default window and weights: 3180 us -> 1837 us (17 of 32 lanes
+// were active before).
+//
 // Summation order per pixel is therefore the reference's (increasing slice index). With an Ewald
 // sphere (curved slices) nothing is culled. The w-windowed form sums the w offsets in registers (in w order)
 // rather than zero-filling and adding atomically; each offset re-samples the virtual volume at the
 // z-shifted frequency.
 #include "fp_args.cuh"
+#include "fp_slice_taps.cuh"
+
+#include <type_traits>
 
 namespace nb {
 namespace {
@@ -47,25 +58,38 @@ __device__ __forceinline__ bool patch_reaches(const float3 n, const Patch& p, co
     return fabsf(centre) <= fb + half + 1e-5f * (1.f + fabsf(centre) + half);
 }
 
-// Six CTAs per SM for the LINEAR and NEAREST instantiations (40 registers, small spills; five fit
-// before): 4096 -> 256 slices at 256^3, 19.75-19.87 -> 15.95-16.10 ms on two boxes. The wider windows
-// keep the compiler's choice.
-template<int I>
-constexpr int insert_extract_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 6 : 1; }
+// One warp's queue of (pixel, slice) pairs: a ring of two halves, evaluated half by half.
+struct PairQueue {
+    unsigned entry[64];   // slice index within the pass << 5 | pixel's lane
+    float fz[64];         // the pixel's distance to the slice
+    float2 value[32];     // of the half evaluated last
+    float weight[32];
+};
 
-template<int I, bool IN_C, bool OUT_C>
+// Whether the pairs take the short arithmetic: Mat33 rotations without scaling or curvature and, for
+// LINEAR, slices that LinearCell can read.
+template<int I>
+bool use_lean(const ProjArgs& a) {
+    return a.rot.kind == 2 && a.scale.kind == 0 && !a.ews.on && (I != I_LINEAR || linear_slices(a));
+}
+
+template<int I>
+constexpr int insert_extract_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 5 : 1; }
+
+template<int I, bool IN_C, bool OUT_C, bool LEAN>
 __global__ void __launch_bounds__(IE_THREADS, insert_extract_min_ctas<I>())
 insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per_slice, int64_t n_tiles) {
     __shared__ int s_list[IE_LIST];
     __shared__ int s_warp_count[IE_THREADS / 32];
     __shared__ float s_box[4][IE_THREADS / 32];
+    __shared__ PairQueue s_queue[IE_THREADS / 32];
 
     const int wp = a.slice_w / 2 + 1;
     const Spectrum2 sp{a.in_h, a.in_w_, a.in_centered, a.in_slice_narrow != 0};
     const bool has_out_w = a.out_w.present;
     const bool has_in_w = a.in_w.present;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool lean = a.rot.kind == 2 && a.scale.kind == 0 && !a.ews.on;
+    PairQueue& queue = s_queue[warp];
 
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const int64_t b = tile / tiles_per_slice;
@@ -149,47 +173,107 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                 if (lane == 0)
                     s_warp_count[warp] = cnt;
                 __syncthreads();
+
+                int filled = 0;               // queued pairs, counted from the pass' start
+                unsigned mine0 = 0, mine1 = 0;  // this lane's pixel's slots of the ring's two halves
+                // Evaluates `n` pairs of a half, one per lane, and adds each pixel's.
+                auto evaluate = [&](int half, int n) {
+                    __syncwarp();
+                    const unsigned entry = queue.entry[half * 32 + lane];  // past n: stale, not used
+                    const float fz = queue.fz[half * 32 + lane];
+                    const int owner = static_cast<int>(entry & 31u);
+                    const float z = __shfl_sync(0xffffffffu, sz, owner);
+                    const float y = __shfl_sync(0xffffffffu, gy, owner);
+                    const float x = __shfl_sync(0xffffffffu, gx, owner);
+                    if (lane < n) {
+                        const int64_t si = super + (entry >> 5);
+                        const float ws = windowed_sinc_fast(fz, a.pfs, a.ifs, a.pfb);
+                        float f0, f1;
+                        if constexpr (LEAN) {
+                            const float* m = xform_ptr(a.rot, si, 12);
+                            f0 = dot3(m[3], m[4], m[5], z, y, x);
+                            f1 = dot3(m[6], m[7], m[8], z, y, x);
+                        } else {
+                            grid2slice(z, y, x, a.scale, a.rot, si, a.ews, f0, f1);
+                        }
+                        const float q0 = mul(f0, a.f_in0), q1 = mul(f1, a.f_in1);
+                        float iw = ws;
+                        if constexpr (LEAN && I == I_LINEAR) {
+                            using T = typename std::conditional<IN_C, float2, float>::type;
+                            const LinearCell cell(sp, q0, q1);
+                            queue.value[lane] = cmul(cell.read(static_cast<const T*>(a.in.data) + si * a.in.s0,
+                                                               static_cast<int>(a.in.s1), static_cast<int>(a.in.s2)), ws);
+                            if (has_in_w)
+                                iw = mul(cell.read(static_cast<const float*>(a.in_w.data) + si * a.in_w.s0,
+                                                   static_cast<int>(a.in_w.s1), static_cast<int>(a.in_w.s2)).x, ws);
+                        } else {
+                            queue.value[lane] = cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, si, q0, q1), ws);
+                            if (has_in_w)
+                                iw = mul(interp_spectrum_2d<I, false>(a.in_w, sp, si, q0, q1).x, ws);
+                        }
+                        queue.weight[lane] = iw;
+                    }
+                    __syncwarp();
+                    unsigned slots = half ? mine1 : mine0;
+                    while (slots) {
+                        const int j = __ffs(slots) - 1;
+                        slots &= slots - 1u;
+                        value = cadd(value, queue.value[j]);
+                        weight = add(weight, queue.weight[j]);
+                    }
+                    if (half)
+                        mine1 = 0;
+                    else
+                        mine0 = 0;
+                };
+
                 for (int region = 0; warp_valid && region < IE_THREADS / 32; ++region) {
                     const int count = s_warp_count[region];
                     const int* list = s_list + region * IE_REGION;
                     for (int g = 0; g < count; g += 32) {
                         const int k = g + lane;
-                        const bool wkeep = k < count &&
-                                           (!cull || patch_reaches(rotation_row0(a.rot, super + list[k]), patch, wbox,
-                                                                   off, a.fb));
+                        const int listed = k < count ? list[k] : 0;
+                        float3 n = make_float3(0.f, 0.f, 0.f);
+                        bool wkeep = k < count;
+                        if (wkeep && (LEAN || cull))
+                            n = rotation_row0(a.rot, super + listed);
+                        if (wkeep && cull)
+                            wkeep = patch_reaches(n, patch, wbox, off, a.fb);
                         unsigned todo = __ballot_sync(0xffffffffu, wkeep);
                         while (todo) {
                             const int j = __ffs(todo) - 1;
                             todo &= todo - 1u;
-                            if (!in_cut)
-                                continue;
-                            const int64_t si = super + list[g + j];
-                            float f0, f1, fz;
-                            if (lean) {
-                                // grid2slice's Mat33 rows, the distance to the plane first: the in-plane
-                                // rows are only needed inside the window (same products and sums).
-                                const float* m = xform_ptr(a.rot, si, 12);
-                                fz = dot3(m[0], m[1], m[2], sz, gy, gx);
-                                if (!(fabsf(fz) < a.fb))
-                                    continue;
-                                f0 = dot3(m[3], m[4], m[5], sz, gy, gx);
-                                f1 = dot3(m[6], m[7], m[8], sz, gy, gx);
+                            const int index = __shfl_sync(0xffffffffu, listed, j);
+                            float fz;
+                            if constexpr (LEAN) {
+                                const float n0 = __shfl_sync(0xffffffffu, n.x, j);
+                                const float n1 = __shfl_sync(0xffffffffu, n.y, j);
+                                const float n2 = __shfl_sync(0xffffffffu, n.z, j);
+                                fz = dot3(n0, n1, n2, sz, gy, gx);
                             } else {
-                                fz = grid2slice(sz, gy, gx, a.scale, a.rot, si, a.ews, f0, f1);
+                                float f0, f1;
+                                fz = grid2slice(sz, gy, gx, a.scale, a.rot, super + index, a.ews, f0, f1);
                             }
-                            if (fabsf(fz) < a.fb) {
-                                const float ws = windowed_sinc_fast(fz, a.pfs, a.ifs, a.pfb);
-                                const float q0 = mul(f0, a.f_in0), q1 = mul(f1, a.f_in1);
-                                value = cadd(value, cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, si, q0, q1), ws));
-                                if (has_in_w)
-                                    weight = add(weight,
-                                                 mul(interp_spectrum_2d<I, false>(a.in_w, sp, si, q0, q1).x, ws));
+                            const bool inside = in_cut && fabsf(fz) < a.fb;
+                            const unsigned ballot = __ballot_sync(0xffffffffu, inside);
+                            if (inside) {
+                                const int slot = (filled + __popc(ballot & ((1u << lane) - 1u))) & 63;
+                                queue.entry[slot] = static_cast<unsigned>(index) << 5 | static_cast<unsigned>(lane);
+                                queue.fz[slot] = fz;
+                                if (slot < 32)
+                                    mine0 |= 1u << slot;
                                 else
-                                    weight = add(weight, ws);
+                                    mine1 |= 1u << (slot - 32);
                             }
+                            const int before = filled >> 5;
+                            filled += __popc(ballot);
+                            if (filled >> 5 != before)  // at most 32 pairs were added: one half is full
+                                evaluate(before & 1, 32);
                         }
                     }
                 }
+                if (filled & 31)
+                    evaluate((filled >> 5) & 1, filled & 31);
                 __syncthreads();
             }
 
@@ -257,7 +341,10 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
         return cudaSuccess;
     const int64_t max_grid = static_cast<int64_t>(sm_count()) * 8 * 16;
     const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    insert_extract_kernel<I, IN_C, OUT_C><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
+    if (use_lean<I>(a))
+        insert_extract_kernel<I, IN_C, OUT_C, true><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
+    else
+        insert_extract_kernel<I, IN_C, OUT_C, false><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
     return cudaGetLastError();
 }
 

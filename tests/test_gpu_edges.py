@@ -61,6 +61,18 @@ def test_linear_insertion(kw, scatter):
     _check(default_case("insert", **{"seed": 704, **kw}), 1e-5, scatter=scatter)
 
 
+# The pair queue: fewer pairs than a half, halves that fill exactly and by many slices, a second pass of the
+# input slices (4096 each), the general rotation, windows over the whole slice, w offsets.
+@pytest.mark.parametrize("kw", [dict(n=12, nslices=1, nout=2), dict(n=10, nslices=4200, nout=1, out_w=True),
+                                dict(n=33, nslices=64, nout=3, sinc=(0.03, 1.0), out_w=True, in_w=True),
+                                dict(n=20, nslices=40, nout=3, rot="quat", scale=True, sinc=(0.02, 0.2), out_w=True),
+                                dict(n=20, nslices=40, nout=2, sinc=(0.02, 0.1), w_sinc=(0.05, 0.2), out_w=True),
+                                dict(n=18, nslices=40, nout=2, in_dt="f32", out_dt="f32", interp="nearest")],
+                         ids=["few", "passes", "wide", "general", "w-window", "nearest"])
+def test_pair_queue(kw):
+    _check(default_case("insert_extract", **{"remap": "h2h", "seed": 705, **kw}), 1e-5)
+
+
 # LINEAR extraction: several slices per CTA with a shorter last group, rows past the slice, cells at the
 # edges of the volume and the non-centered wrap, with and without the pair copy.
 @pytest.mark.parametrize("remap", ["h2h", "hc2hc"])

@@ -317,10 +317,24 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
     return r;
 }
 
-// Two single-precision fused multiply-adds, each rounded as fmaf, in one instruction.
+// Two single-precision operations in one instruction, each rounded as fmaf (__fmul_rn, __fadd_rn). Unlike the
+// scalar intrinsics, a packed product that only feeds a packed sum is fused with it (observed with CUDA
+// 12.9), so where products have to be rounded on their own they are made by mul() and packed for the sums.
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 

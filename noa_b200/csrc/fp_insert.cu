@@ -172,13 +172,15 @@ insert_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int nbx) {
     }
 }
 
-// The LINEAR insertion of Mat33 rotations without scaling or curvature, from slices whose inner offsets fit
-// 32 bits: insert_kernel's sum, term for term in the same order, for few instructions per (voxel, slice)
+// The LINEAR insertion of Mat33 rotations without scaling or curvature, from slices with adjacent columns:
+// insert_kernel's sum, term for term in the same order, for few instructions per (voxel, slice)
 // pair, which is what bounds it: 400 slices
-// into 512^3 with half-width 6 and weights 6074 us -> 3803 us (insert_kernel issues at 87 % of its rate).
+// into 512^3 with half-width 6 and weights 6074 us -> 3083 us (insert_kernel issues at 87 % of its rate; 3803
+// us with the window and the coordinates of one voxel at a time).
 //
 // A thread owns LIN_PZ voxels along z: the products of a slice's matrix with the voxels' y and x
-// frequencies are shared by them, so a voxel costs one product and two sums per row of the matrix. A
+// frequencies are shared by them, so a voxel costs one product and two sums per row of the matrix, and the
+// sums and the window of two voxels run in packed operations. A
 // slice's matrix and base pointer are staged as three 16-byte words, the test of the cull is the exact
 // interval of n . f over the brick's box, and a chunk of the list holds twice as many slices as the CTA
 // has threads (half the barriers).
@@ -188,19 +190,7 @@ constexpr int LIN_THREADS = LIN_Z / LIN_PZ * LIN_Y * LIN_X;  // 128; a warp cove
 constexpr int LIN_CHUNK = 2 * LIN_THREADS;                   // slices culled per pass
 constexpr int LIN_WARPS = LIN_THREADS / 32;
 
-// Centre and half extent of the frequencies of indices [first, first + count) of one axis, in fftfreq.
-__device__ __forceinline__ float2 axis_box(bool half_axis, bool centered, int first, int count, int n, float target) {
-    float mn = 3.4e38f, mx = -3.4e38f;
-    for (int k = 0; k < count && first + k < n; ++k) {
-        const int f = half_axis ? first + k : index2frequency(centered, first + k, n);
-        const float ff = static_cast<float>(f) / target;
-        mn = fminf(mn, ff);
-        mx = fmaxf(mx, ff);
-    }
-    return make_float2(0.5f * (mn + mx), 0.5f * (mx - mn));
-}
-
-template<bool IN_C, bool OUT_C>
+template<bool IN_C, bool OUT_C, typename Idx>
 __global__ void __launch_bounds__(LIN_THREADS, 8)
 insert_linear_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int nbx) {
     using T = typename std::conditional<IN_C, float2, float>::type;
@@ -213,7 +203,8 @@ insert_linear_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int n
     const Spectrum2 sp{a.slice_h, a.slice_w, a.in_centered, true};
     const bool has_out_w = a.out_w.present;
     const bool has_in_w = has_out_w && a.in_w.present;
-    const int s1 = static_cast<int>(a.in.s1), s2 = static_cast<int>(a.in.s2);
+    const Idx s1 = static_cast<Idx>(a.in.s1);
+    const WindowPair window_of(a);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = tid % LIN_X, ty = (tid / LIN_X) % LIN_Y, tz = tid / (LIN_X * LIN_Y) * LIN_PZ;
     const int64_t n_bricks = static_cast<int64_t>(nbz) * nby * nbx;
@@ -238,11 +229,22 @@ insert_linear_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int n
         if (!__syncthreads_or(active))
             continue;
 
-        // The brick's box; the non-centered layout wraps, so its extents are scanned, not assumed.
-        if (tid < 3)
-            s_box[tid] = axis_box(tid == 2, vc, tid == 0 ? bz * LIN_Z : tid == 1 ? by * LIN_Y : bx * LIN_X, 8,
-                                  tid == 0 ? D : tid == 1 ? H : WP,
-                                  tid == 0 ? a.target0 : tid == 1 ? a.target1 : a.target2);
+        // The brick's box, centre and half extent per axis; the non-centered layout wraps, so its extents
+        // are the smallest and largest of the indices', 8 lanes per axis.
+        if (warp == 0) {
+            const int axis = lane >> 3, first = axis == 0 ? bz * LIN_Z : axis == 1 ? by * LIN_Y : bx * LIN_X;
+            const int n = axis == 0 ? D : axis == 1 ? H : WP, i = min(first + (lane & 7), n - 1);
+            const float f = static_cast<float>(axis < 2 ? index2frequency(vc, i, n) : i) /
+                            (axis == 0 ? a.target0 : axis == 1 ? a.target1 : a.target2);
+            float mn = f, mx = f;
+#pragma unroll
+            for (int o = 4; o > 0; o /= 2) {
+                mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            if ((lane & 7) == 0 && axis < 3)
+                s_box[axis] = make_float2(0.5f * (mn + mx), 0.5f * (mx - mn));
+        }
         __syncthreads();
         const float2 box0 = s_box[0], box1 = s_box[1], box2 = s_box[2];
 
@@ -295,13 +297,15 @@ insert_linear_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int n
                 for (int s = 0; s < count; ++s) {
                     const float4 r0 = s_row[0][s];
                     const float y0 = mul(r0.y, fy), x0 = mul(r0.z, fx);
-                    float zz[LIN_PZ];
-                    bool near = false;
+                    unsigned long long zz[LIN_PZ / 2];
+                    unsigned near = 0;  // voxels within the window
 #pragma unroll
-                    for (int k = 0; k < LIN_PZ; ++k) {
-                        zz[k] = add(add(mul(r0.x, fz[k]), y0), x0);
-                        near = near || fabsf(zz[k]) <= a.fb;
+                    for (int h = 0; h < LIN_PZ / 2; ++h) {
+                        zz[h] = add2(add2(pack2(mul(r0.x, fz[2 * h]), mul(r0.x, fz[2 * h + 1])), pack2(y0, y0)), pack2(x0, x0));
+                        const float2 z = unpack2(zz[h]);
+                        near |= (fabsf(z.x) <= a.fb ? 1u << 2 * h : 0u) | (fabsf(z.y) <= a.fb ? 2u << 2 * h : 0u);
                     }
+                    near &= active;
                     if (!near)
                         continue;
                     const float4 r1 = s_row[1][s], r2 = s_row[2][s];
@@ -309,20 +313,33 @@ insert_linear_kernel(const __grid_constant__ ProjArgs a, int nbz, int nby, int n
                     const T* base = reinterpret_cast<const T*>(static_cast<uint64_t>(__float_as_uint(r1.w)) |
                                                                static_cast<uint64_t>(__float_as_uint(r2.w)) << 32);
 #pragma unroll
-                    for (int k = 0; k < LIN_PZ; ++k) {
-                        if (!(fabsf(zz[k]) <= a.fb) || !((active >> k) & 1u))
+                    for (int h = 0; h < LIN_PZ / 2; ++h) {
+                        if (!(near & (3u << 2 * h)))
                             continue;
-                        const float window = windowed_sinc_fast(zz[k], a.pfs, a.ifs, a.pfb);
-                        const float q0 = mul(add(add(mul(r1.x, fz[k]), y1), x1), a.f_slice0);
-                        const float q1 = mul(add(add(mul(r2.x, fz[k]), y2), x2), a.f_slice1);
-                        const LinearCell cell(sp, q0, q1);
-                        value[k] = cadd(value[k], cmul(cell.read(base, s1, s2), window));
-                        if (has_in_w) {
-                            const float* base_w = static_cast<const float*>(a.in_w.data) + __float_as_int(r0.w) * a.in_w.s0;
-                            const float iw = cell.read(base_w, static_cast<int>(a.in_w.s1), static_cast<int>(a.in_w.s2)).x;
-                            weights[k] = add(weights[k], mul(iw, window));
-                        } else {
-                            weights[k] = add(weights[k], window);
+                        const float2 window = window_of(zz[h]);
+                        const float za = fz[2 * h], zb = fz[2 * h + 1];
+                        const float2 q0 = unpack2(mul2(add2(add2(pack2(mul(r1.x, za), mul(r1.x, zb)), pack2(y1, y1)), pack2(x1, x1)),
+                                                       pack2(a.f_slice0, a.f_slice0)));
+                        const float2 q1 = unpack2(mul2(add2(add2(pack2(mul(r2.x, za), mul(r2.x, zb)), pack2(y2, y2)), pack2(x2, x2)),
+                                                       pack2(a.f_slice1, a.f_slice1)));
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int k = 2 * h + e;
+                            if (!((near >> k) & 1u))
+                                continue;
+                            const float w = e ? window.y : window.x;
+                            const T v = slice_value(base, sp, s1, e ? q0.y : q0.x, e ? q1.y : q1.x);
+                            if constexpr (IN_C)
+                                value[k] = cfma(v, w, value[k]);
+                            else
+                                value[k].x = fmaf(v, w, value[k].x);
+                            if (has_in_w) {
+                                const float* base_w = static_cast<const float*>(a.in_w.data) + __float_as_int(r0.w) * a.in_w.s0;
+                                const LinearCell cell(sp, e ? q0.y : q0.x, e ? q1.y : q1.x);
+                                weights[k] = fmaf(cell.read(base_w, static_cast<Idx>(a.in_w.s1), static_cast<Idx>(a.in_w.s2)).x, w, weights[k]);
+                            } else {
+                                weights[k] += w;
+                            }
                         }
                     }
                 }
@@ -351,7 +368,11 @@ cudaError_t launch_linear(const ProjArgs& a, cudaStream_t stream) {
     if (n == 0)
         return cudaSuccess;
     const int64_t max_grid = int64_t(1) << 30;
-    insert_linear_kernel<IN_C, OUT_C><<<static_cast<unsigned>(n < max_grid ? n : max_grid), LIN_THREADS, 0, stream>>>(a, nbz, nby, nbx);
+    const unsigned grid = static_cast<unsigned>(n < max_grid ? n : max_grid);
+    if (a.in_slice_narrow)
+        insert_linear_kernel<IN_C, OUT_C, int><<<grid, LIN_THREADS, 0, stream>>>(a, nbz, nby, nbx);
+    else
+        insert_linear_kernel<IN_C, OUT_C, int64_t><<<grid, LIN_THREADS, 0, stream>>>(a, nbz, nby, nbx);
     return cudaGetLastError();
 }
 

@@ -114,15 +114,15 @@ insert_scatter_kernel(const __grid_constant__ ProjArgs a, void* __restrict__ acc
     }
 }
 
-// The LINEAR form for Mat33 rotations without scaling, from slices whose inner offsets fit 32 bits:
+// The LINEAR form for Mat33 rotations without scaling, from slices with adjacent columns:
 // insert_scatter_kernel's terms for few instructions per (voxel, slice) pair, which is what bounds it:
-// 500 slices into 256^3 with half-width 6 and weights 2620 us -> 1676 us.
+// 500 slices into 256^3 with half-width 6 and weights 2620 us -> 1389 us (1676 us one voxel at a time).
 //
 // The axis that the columns run along is a compile-time constant (the slice picks one of three bodies), so
 // the products of the matrix with the column's two fixed frequencies, and the accumulator offset, are
 // computed once per column; the frequencies come from a table per CTA instead of divisions; and the k
 // range is widened by its rounding error instead of a whole voxel each side.
-template<int AX, bool IN_C, bool W>
+template<int AX, bool IN_C, bool W, typename Idx>
 __device__ __forceinline__ void scatter_column(const ProjArgs& a, void* acc, const float* freq, int col, int64_t slice,
                                                const float* m) {
     constexpr int P = AX == 0 ? 1 : 0, Q = AX == 2 ? 1 : 2;  // the column's fixed axes, Q fastest
@@ -153,38 +153,61 @@ __device__ __forceinline__ void scatter_column(const ProjArgs& a, void* acc, con
     const auto index = [vc](int k, int n) { return frequency2index(vc, k, n); };
     // Offset of the column; x frequencies are their indices.
     const int offset = index(lo[P] + ip, extent[P]) * stride[P] + (Q == 2 ? iq : index(lo[Q] + iq, extent[Q]) * stride[Q]);
-    const int s1 = static_cast<int>(a.in.s1), s2 = static_cast<int>(a.in.s2);
+    const Idx s1 = static_cast<Idx>(a.in.s1);
+    const WindowPair window_of(a);
     using T = typename std::conditional<IN_C, float2, float>::type;
     const T* base = static_cast<const T*>(a.in.data) + slice * a.in.s0;
     const float* base_w = has_in_w ? static_cast<const float*>(a.in_w.data) + slice * a.in_w.s0 : nullptr;
-    // v0 z + v1 y + v2 x summed in that order, the terms of the fixed axes given.
-    const auto dot = [](float run, float p, float q) {
+    // v0 z + v1 y + v2 x summed in that order, the terms of the fixed axes given; for two voxels at a time.
+    const auto both = [](float v) { return pack2(v, v); };
+    const auto dot = [both](float c, float f0, float f1, float p, float q) {
+        const unsigned long long run = pack2(mul(c, f0), mul(c, f1));
+        return AX == 0 ? add2(add2(run, both(p)), both(q)) : AX == 1 ? add2(add2(both(p), run), both(q))
+                                                                     : add2(both(add(p, q)), run);
+    };
+    const auto dot3_axis = [](float run, float p, float q) {
         return AX == 0 ? add(add(run, p), q) : AX == 1 ? add(add(p, run), q) : add(add(p, q), run);
     };
     const float pp = mul(fp, fp), qq = mul(fq, fq);
     const float p0 = mul(m[P], fp), q0 = mul(m[Q], fq), p1 = mul(m[3 + P], fp), q1 = mul(m[3 + Q], fq);
     const float p2 = mul(m[6 + P], fp), q2 = mul(m[6 + Q], fq);
-    for (int k = first; k <= last; ++k) {
-        // The gather form's term (fp_insert.cu, FourierProject.hpp:479-518).
-        const float f = fa[k];
-        const float zz = dot(mul(m[AX], f), p0, q0);
-        if (!(fabsf(zz) <= a.fb) || dot(mul(f, f), pp, qq) > a.cutoff_sqd)
+    for (int k = first; k <= last; k += 2) {
+        // The gather form's terms (fp_insert.cu, FourierProject.hpp:479-518).
+        const float f0 = fa[k], f1 = fa[min(k + 1, last)];
+        const unsigned long long zz = dot(m[AX], f0, f1, p0, q0);
+        const float2 z = unpack2(zz);
+        const float sqd0 = dot3_axis(mul(f0, f0), pp, qq), sqd1 = dot3_axis(mul(f1, f1), pp, qq);
+        const bool in0 = fabsf(z.x) <= a.fb && !(sqd0 > a.cutoff_sqd);
+        const bool in1 = k < last && fabsf(z.y) <= a.fb && !(sqd1 > a.cutoff_sqd);
+        if (!in0 && !in1)
             continue;
-        const float window = windowed_sinc_fast(zz, a.pfs, a.ifs, a.pfb);
-        const LinearCell cell(sp, mul(dot(mul(m[3 + AX], f), p1, q1), a.f_slice0),
-                              mul(dot(mul(m[6 + AX], f), p2, q2), a.f_slice1));
-        const float2 v = cmul(cell.read(base, s1, s2), window);
-        float w = 0.f;
-        if constexpr (W)
-            w = has_in_w ? mul(cell.read(base_w, static_cast<int>(a.in_w.s1), static_cast<int>(a.in_w.s2)).x, window) : window;
-        acc_red<IN_C, W>(acc, offset + (AX == 2 ? k : index(lo[AX] + k, extent[AX]) * stride[AX]), v, w);
+        const float2 window = window_of(zz);
+        const float2 c0 = unpack2(mul2(dot(m[3 + AX], f0, f1, p1, q1), both(a.f_slice0)));
+        const float2 c1 = unpack2(mul2(dot(m[6 + AX], f0, f1, p2, q2), both(a.f_slice1)));
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            if (!(e ? in1 : in0))
+                continue;
+            float w = e ? window.y : window.x;
+            const float s0 = e ? c0.y : c0.x, s1_ = e ? c1.y : c1.x;
+            float2 v;
+            if constexpr (IN_C)
+                v = cmul(slice_value(base, sp, s1, s0, s1_), w);
+            else
+                v = make_float2(slice_value(base, sp, s1, s0, s1_) * w, 0.f);
+            if (W && has_in_w) {
+                const LinearCell cell(sp, s0, s1_);
+                w = mul(cell.read(base_w, static_cast<Idx>(a.in_w.s1), static_cast<Idx>(a.in_w.s2)).x, w);
+            }
+            acc_red<IN_C, W>(acc, offset + (AX == 2 ? k + e : index(lo[AX] + k + e, extent[AX]) * stride[AX]), v, w);
+        }
     }
 }
 
 // Frequencies of one CTA's table: all indices of the three axes.
 constexpr int SCATTER_TABLE = 8192;
 
-template<bool IN_C, bool W>
+template<bool IN_C, bool W, typename Idx>
 __global__ void __launch_bounds__(SCATTER_THREADS)
 scatter_linear_kernel(const __grid_constant__ ProjArgs a, void* __restrict__ acc) {
     extern __shared__ float s_freq[];
@@ -199,11 +222,11 @@ scatter_linear_kernel(const __grid_constant__ ProjArgs a, void* __restrict__ acc
         const float* m = xform_ptr(a.rot, i, 12);
         const float c0 = fabsf(m[0] / a.target0), c1 = fabsf(m[1] / a.target1), c2 = fabsf(m[2] / a.target2);
         if (c0 >= c1 && c0 >= c2)
-            scatter_column<0, IN_C, W>(a, acc, s_freq, col, i, m);
+            scatter_column<0, IN_C, W, Idx>(a, acc, s_freq, col, i, m);
         else if (c1 >= c2)
-            scatter_column<1, IN_C, W>(a, acc, s_freq, col, i, m);
+            scatter_column<1, IN_C, W, Idx>(a, acc, s_freq, col, i, m);
         else
-            scatter_column<2, IN_C, W>(a, acc, s_freq, col, i, m);
+            scatter_column<2, IN_C, W, Idx>(a, acc, s_freq, col, i, m);
     }
 }
 
@@ -255,7 +278,10 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream, bool& done) {
                         static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
         if (I == I_LINEAR && use_linear_scatter(a)) {
             const size_t table = static_cast<size_t>(D + H + WP) * sizeof(float);
-            scatter_linear_kernel<IN_C, W><<<grid, SCATTER_THREADS, table, stream>>>(a, acc);
+            if (a.in_slice_narrow)
+                scatter_linear_kernel<IN_C, W, int><<<grid, SCATTER_THREADS, table, stream>>>(a, acc);
+            else
+                scatter_linear_kernel<IN_C, W, int64_t><<<grid, SCATTER_THREADS, table, stream>>>(a, acc);
         } else {
             insert_scatter_kernel<I, IN_C, W><<<grid, SCATTER_THREADS, 0, stream>>>(a, acc);
         }

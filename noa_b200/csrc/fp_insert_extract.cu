@@ -6,16 +6,23 @@
 // and without curvature g is linear in the pixel's 2-D frequency, so n_i . g over a box of pixels is an
 // interval known from two dot products (patch_reaches). The slices whose interval over the CTA's box
 // meets the slab are compacted, in increasing order, into shared memory, 4096 at a time, each warp
-// compacting its own range of slice indices so that building the list needs no barrier; each warp then
-// re-tests the whole list against its own box (one candidate per lane) and walks the survivors' ballot
-// in lane order, with no barrier until the next pass.
+// compacting its own range of slice indices so that building the list needs no barrier.
 //
-// A third of the warp's pixels lie within a surviving slice's slab, so the walk only computes the distances
-// to it and queues the (pixel, slice) pairs inside, and the warp evaluates queued pairs 32 at a time, one
-// per lane, whichever pixels they belong to: window and interpolation run with all lanes busy. Each lane
-// keeps the queue slots of its own pixel's pairs as a bit mask and adds their results in slot order.
-// 2000 input to 64 output slices of 256^2, default window and weights: 3180 us -> 1837 us (17 of 32 lanes
-// were active before).
+// Each warp then takes the list 32 slices at a time, one per lane, with no barrier until the next pass. fz is
+// linear along a row of pixels, so a slice's slab covers an interval of each of the warp's four rows
+// (widened by the rounding of the exact test): together a 32-bit mask of pixels. The warp walks the slices
+// whose mask is not empty, queues their (pixel, slice) pairs and evaluates queued pairs 64 at a time, two per
+// lane, whichever pixels they belong to: exact distance, window and interpolation run with all lanes busy,
+// although a third of the pixels lie within any one slice's slab. Each lane keeps the queue slots of its own
+// pixel's pairs as a bit mask and adds their results in slot order. (Every lane evaluating its own pixel of
+// one slice at a time had 17 of 32 lanes active; masks transposed so that each lane walks its own pixel's
+// slices without a queue were 10 % slower, the longest list of 32 setting the pace.)
+//
+// The slices through a pixel grow as 1 / |f|, so the tiles around the origin hold up to 20 times the pairs
+// of the others, and the warp at the origin works for a good part of the launch: tiles are taken in the order
+// of their distance to it, those of all output slices together, so that the long ones start first. 2000
+// input to 64 output slices of 256^2, default window and weights: 3180 us ->
+// 1837 us with a queue filled by exact tests and evaluated 32 pairs at a time -> 1253 us.
 //
 // Summation order per pixel is therefore the reference's (increasing slice index). With an Ewald
 // sphere (curved slices) nothing is culled. The w-windowed form sums the w offsets in registers (in w order)
@@ -58,12 +65,34 @@ __device__ __forceinline__ bool patch_reaches(const float3 n, const Patch& p, co
     return fabsf(centre) <= fb + half + 1e-5f * (1.f + fabsf(centre) + half);
 }
 
+// The pixels of a warp's 4 x 8 patch (bit 8 row + column) that slice n may reach, fz being linear along a row.
+// `rows`: the rows' 2-D frequencies; `first`, `step`: the first column's frequency and the columns' spacing.
+__device__ __forceinline__ unsigned patch_mask(const float3 n, const Patch& p, const float (&rows)[4], float first,
+                                               float step, float off, float fb) {
+    const float al = n.x * p.gv0 + n.y * p.gv1 + n.z * p.gv2;
+    const float be = n.x * p.gu0 + n.y * p.gu1 + n.z * p.gu2;
+    const float shift = n.x * off;
+    const float reach = fb + 1e-5f * (1.f + fabsf(al) + fabsf(be) + fabsf(shift));
+    const float inv = 1.f / (be * step);  // infinite for a slice parallel to the rows: all or nothing below
+    unsigned mask = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float start = al * rows[r] + be * first + shift;
+        const float a = (-reach - start) * inv, b = (reach - start) * inv;
+        // Clamped before the conversions (NaN included: then the whole row, and the exact test decides).
+        const int lo = __float2int_ru(fminf(fmaxf(fminf(a, b) - 1e-3f, 0.f), 8.f));
+        const int hi = __float2int_rd(fmaxf(fminf(fmaxf(a, b) + 1e-3f, 7.f), -1.f));
+        mask |= ((2u << hi) - (1u << lo) & (hi >= lo ? 0xffu : 0u)) << 8 * r;
+    }
+    return mask;
+}
+
 // One warp's queue of (pixel, slice) pairs: a ring of two halves, evaluated half by half.
+constexpr int IE_HALF = 64;
 struct PairQueue {
-    unsigned entry[64];   // slice index within the pass << 5 | pixel's lane
-    float fz[64];         // the pixel's distance to the slice
-    float2 value[32];     // of the half evaluated last
-    float weight[32];
+    unsigned entry[2 * IE_HALF];   // slice index within the pass << 5 | pixel's lane
+    float2 value[IE_HALF];         // of the half evaluated last
+    float weight[IE_HALF];
 };
 
 // Whether the pairs take the short arithmetic: Mat33 rotations without scaling or curvature and, for
@@ -74,9 +103,9 @@ bool use_lean(const ProjArgs& a) {
 }
 
 template<int I>
-constexpr int insert_extract_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 5 : 1; }
+constexpr int insert_extract_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 4 : 1; }
 
-template<int I, bool IN_C, bool OUT_C, bool LEAN>
+template<int I, bool IN_C, bool OUT_C, bool LEAN, typename Idx = int>
 __global__ void __launch_bounds__(IE_THREADS, insert_extract_min_ctas<I>())
 insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per_slice, int64_t n_tiles) {
     __shared__ int s_list[IE_LIST];
@@ -90,11 +119,17 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
     const bool has_in_w = a.in_w.present;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     PairQueue& queue = s_queue[warp];
+    const WindowPair window_of(a);
 
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int64_t b = tile / tiles_per_slice;
-        const int t = static_cast<int>(tile - b * tiles_per_slice);
-        const int ty = t / ntx, tx = t - ty * ntx;
+        // The tile's place by distance to the origin (column of tiles, then rows alternately below and above
+        // the origin's), all output slices of one place together.
+        const int place = static_cast<int>(tile / a.n_slices);
+        const int64_t b = tile - place * a.n_slices;
+        const int nty = tiles_per_slice / ntx;
+        const int tx = place / nty, k_row = place - tx * nty;
+        const int origin = a.out_centered ? a.slice_h / 2 / IE_TILE : 0;
+        const int ty = (origin + (k_row & 1 ? nty - (k_row + 1) / 2 : k_row / 2)) % nty;
         const int py = ty * IE_TILE + (warp >> 1) * 4 + (lane >> 3);
         const int pu = tx * IE_TILE + (warp & 1) * 8 + (lane & 7);
         const bool valid = py < a.slice_h && pu < wp;
@@ -124,9 +159,13 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                 s_box[2 + ax][warp] = bmax[ax];
             }
         }
-        // After the butterfly every lane holds its warp's box.
         const bool warp_valid = __any_sync(0xffffffffu, valid);
-        const Box2 wbox = Box2::of(bmin[0], bmax[0], bmin[1], bmax[1]);
+        // The warp's rows and columns (the non-centered layout wraps between rows, not along them).
+        float rows[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            rows[r] = __shfl_sync(0xffffffffu, pf0, 8 * r);
+        const float first = __shfl_sync(0xffffffffu, static_cast<float>(pu), 0) / a.f_slice1;
         __syncthreads();
         float lo[2], hi[2];
 #pragma unroll
@@ -153,6 +192,7 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
             const float off = a.wsize > 1 ? div(static_cast<float>(w - a.wsize / 2), a.vz) : 0.f;
             const float sz = a.wsize > 1 ? add(gz, off) : gz;
             const bool in_cut = valid && dot3(sz, gy, gx, sz, gy, gx) <= a.cutoff_sqd;
+            const unsigned cut_mask = __ballot_sync(0xffffffffu, in_cut);
             float2 value = make_float2(0.f, 0.f);
             float weight = 0.f;
 
@@ -174,50 +214,83 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                     s_warp_count[warp] = cnt;
                 __syncthreads();
 
-                int filled = 0;               // queued pairs, counted from the pass' start
-                unsigned mine0 = 0, mine1 = 0;  // this lane's pixel's slots of the ring's two halves
-                // Evaluates `n` pairs of a half, one per lane, and adds each pixel's.
+                int filled = 0;                           // queued pairs, counted from the pass' start
+                unsigned long long mine0 = 0, mine1 = 0;  // this lane's pixel's slots of the ring's two halves
+                // Evaluates `n` pairs of a half, two per lane, and adds each pixel's.
                 auto evaluate = [&](int half, int n) {
                     __syncwarp();
-                    const unsigned entry = queue.entry[half * 32 + lane];  // past n: stale, not used
-                    const float fz = queue.fz[half * 32 + lane];
-                    const int owner = static_cast<int>(entry & 31u);
-                    const float z = __shfl_sync(0xffffffffu, sz, owner);
-                    const float y = __shfl_sync(0xffffffffu, gy, owner);
-                    const float x = __shfl_sync(0xffffffffu, gx, owner);
-                    if (lane < n) {
-                        const int64_t si = super + (entry >> 5);
-                        const float ws = windowed_sinc_fast(fz, a.pfs, a.ifs, a.pfb);
+                    int64_t si[2];
+                    float q0[2], q1[2], fz[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int at = lane + 32 * e;
+                        // past n: stale, read as the first pair and not stored
+                        const unsigned entry = queue.entry[half * IE_HALF + (at < n ? at : 0)];
+                        const int owner = static_cast<int>(entry & 31u);
+                        const float z = __shfl_sync(0xffffffffu, sz, owner);
+                        const float y = __shfl_sync(0xffffffffu, gy, owner);
+                        const float x = __shfl_sync(0xffffffffu, gx, owner);
+                        si[e] = super + (entry >> 5);
                         float f0, f1;
                         if constexpr (LEAN) {
-                            const float* m = xform_ptr(a.rot, si, 12);
+                            const float* m = xform_ptr(a.rot, si[e], 12);
+                            fz[e] = dot3(m[0], m[1], m[2], z, y, x);
                             f0 = dot3(m[3], m[4], m[5], z, y, x);
                             f1 = dot3(m[6], m[7], m[8], z, y, x);
                         } else {
-                            grid2slice(z, y, x, a.scale, a.rot, si, a.ews, f0, f1);
+                            fz[e] = grid2slice(z, y, x, a.scale, a.rot, si[e], a.ews, f0, f1);
                         }
-                        const float q0 = mul(f0, a.f_in0), q1 = mul(f1, a.f_in1);
-                        float iw = ws;
-                        if constexpr (LEAN && I == I_LINEAR) {
-                            using T = typename std::conditional<IN_C, float2, float>::type;
-                            const LinearCell cell(sp, q0, q1);
-                            queue.value[lane] = cmul(cell.read(static_cast<const T*>(a.in.data) + si * a.in.s0,
-                                                               static_cast<int>(a.in.s1), static_cast<int>(a.in.s2)), ws);
-                            if (has_in_w)
-                                iw = mul(cell.read(static_cast<const float*>(a.in_w.data) + si * a.in_w.s0,
-                                                   static_cast<int>(a.in_w.s1), static_cast<int>(a.in_w.s2)).x, ws);
-                        } else {
-                            queue.value[lane] = cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, si, q0, q1), ws);
-                            if (has_in_w)
-                                iw = mul(interp_spectrum_2d<I, false>(a.in_w, sp, si, q0, q1).x, ws);
+                        q0[e] = mul(f0, a.f_in0);
+                        q1[e] = mul(f1, a.f_in1);
+                    }
+                    float2 iv[2] = {};
+                    float iw[2] = {};
+                    if constexpr (LEAN && I == I_LINEAR) {
+                        using T = typename std::conditional<IN_C, float2, float>::type;
+                        const float2 window = window_of(pack2(fz[0], fz[1]));
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (!(fabsf(fz[e]) < a.fb))
+                                continue;
+                            iw[e] = e ? window.y : window.x;
+                            const T* base = static_cast<const T*>(a.in.data) + si[e] * a.in.s0;
+                            if constexpr (IN_C)
+                                iv[e] = cmul(slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]), iw[e]);
+                            else
+                                iv[e].x = slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]) * iw[e];
+                            if (has_in_w) {
+                                const LinearCell cell(sp, q0[e], q1[e]);
+                                iw[e] = mul(cell.read(static_cast<const float*>(a.in_w.data) + si[e] * a.in_w.s0,
+                                                      static_cast<Idx>(a.in_w.s1), static_cast<Idx>(a.in_w.s2)).x, iw[e]);
+                            }
                         }
-                        queue.weight[lane] = iw;
+                    } else {
+#pragma unroll 1
+                        for (int e = 0; e < 2; ++e) {
+                            const float f = e ? fz[1] : fz[0], c0 = e ? q0[1] : q0[0], c1 = e ? q1[1] : q1[0];
+                            const int64_t i = e ? si[1] : si[0];
+                            if (!(fabsf(f) < a.fb))
+                                continue;
+                            float w1 = windowed_sinc_fast(f, a.pfs, a.ifs, a.pfb);
+                            const float2 v1 = cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, i, c0, c1), w1);
+                            if (has_in_w)
+                                w1 = mul(interp_spectrum_2d<I, false>(a.in_w, sp, i, c0, c1).x, w1);
+                            (e ? iv[1] : iv[0]) = v1;
+                            (e ? iw[1] : iw[0]) = w1;
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (lane + 32 * e < n) {
+                            queue.value[lane + 32 * e] = iv[e];
+                            queue.weight[lane + 32 * e] = iw[e];
+                        }
                     }
                     __syncwarp();
-                    unsigned slots = half ? mine1 : mine0;
+                    unsigned long long slots = half ? mine1 : mine0;
                     while (slots) {
-                        const int j = __ffs(slots) - 1;
-                        slots &= slots - 1u;
+                        const int j = __ffsll(static_cast<long long>(slots)) - 1;
+                        slots &= slots - 1;
                         value = cadd(value, queue.value[j]);
                         weight = add(weight, queue.weight[j]);
                     }
@@ -233,47 +306,33 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                     for (int g = 0; g < count; g += 32) {
                         const int k = g + lane;
                         const int listed = k < count ? list[k] : 0;
-                        float3 n = make_float3(0.f, 0.f, 0.f);
-                        bool wkeep = k < count;
-                        if (wkeep && (LEAN || cull))
-                            n = rotation_row0(a.rot, super + listed);
-                        if (wkeep && cull)
-                            wkeep = patch_reaches(n, patch, wbox, off, a.fb);
-                        unsigned todo = __ballot_sync(0xffffffffu, wkeep);
+                        unsigned mask = k < count ? cut_mask : 0u;
+                        if (mask && cull)
+                            mask &= patch_mask(rotation_row0(a.rot, super + listed), patch, rows, first, 1.f / a.f_slice1,
+                                               off, a.fb);
+                        unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
                         while (todo) {
                             const int j = __ffs(todo) - 1;
                             todo &= todo - 1u;
                             const int index = __shfl_sync(0xffffffffu, listed, j);
-                            float fz;
-                            if constexpr (LEAN) {
-                                const float n0 = __shfl_sync(0xffffffffu, n.x, j);
-                                const float n1 = __shfl_sync(0xffffffffu, n.y, j);
-                                const float n2 = __shfl_sync(0xffffffffu, n.z, j);
-                                fz = dot3(n0, n1, n2, sz, gy, gx);
-                            } else {
-                                float f0, f1;
-                                fz = grid2slice(sz, gy, gx, a.scale, a.rot, super + index, a.ews, f0, f1);
-                            }
-                            const bool inside = in_cut && fabsf(fz) < a.fb;
-                            const unsigned ballot = __ballot_sync(0xffffffffu, inside);
-                            if (inside) {
-                                const int slot = (filled + __popc(ballot & ((1u << lane) - 1u))) & 63;
+                            const unsigned pixels = __shfl_sync(0xffffffffu, mask, j);
+                            if ((pixels >> lane) & 1u) {
+                                const int slot = (filled + __popc(pixels & ((1u << lane) - 1u))) & (2 * IE_HALF - 1);
                                 queue.entry[slot] = static_cast<unsigned>(index) << 5 | static_cast<unsigned>(lane);
-                                queue.fz[slot] = fz;
-                                if (slot < 32)
-                                    mine0 |= 1u << slot;
+                                if (slot < IE_HALF)
+                                    mine0 |= 1ull << slot;
                                 else
-                                    mine1 |= 1u << (slot - 32);
+                                    mine1 |= 1ull << (slot - IE_HALF);
                             }
-                            const int before = filled >> 5;
-                            filled += __popc(ballot);
-                            if (filled >> 5 != before)  // at most 32 pairs were added: one half is full
-                                evaluate(before & 1, 32);
+                            const int before = filled / IE_HALF;
+                            filled += __popc(pixels);
+                            if (filled / IE_HALF != before)  // at most 32 pairs were added: one half is full
+                                evaluate(before & 1, IE_HALF);
                         }
                     }
                 }
-                if (filled & 31)
-                    evaluate((filled >> 5) & 1, filled & 31);
+                if (filled % IE_HALF)
+                    evaluate(filled / IE_HALF & 1, filled % IE_HALF);
                 __syncthreads();
             }
 
@@ -341,7 +400,14 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
         return cudaSuccess;
     const int64_t max_grid = static_cast<int64_t>(sm_count()) * 8 * 16;
     const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    if (use_lean<I>(a))
+    const bool lean = use_lean<I>(a);
+    if constexpr (I == I_LINEAR) {
+        if (lean && !a.in_slice_narrow) {
+            insert_extract_kernel<I, IN_C, OUT_C, true, int64_t><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
+            return cudaGetLastError();
+        }
+    }
+    if (lean)
         insert_extract_kernel<I, IN_C, OUT_C, true><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
     else
         insert_extract_kernel<I, IN_C, OUT_C, false><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);

@@ -229,6 +229,19 @@ bool needs_wide(const nb_array* a) {
     return extent >= (int64_t(1) << 31) - 1;
 }
 
+// Whether an array's elements all lie within 4 GiB of its start (true for absent arrays).
+bool spans_bytes32(const nb_array* a) {
+    if (!is_array(a))
+        return true;
+    int64_t extent = 1;
+    for (int i = 0; i < 4; ++i) {
+        if (a->strides[i] >= (int64_t(1) << 32))
+            return false;
+        extent += (a->shape[i] - 1) * a->strides[i];
+    }
+    return extent < (int64_t(1) << 32) / elem_size(a->dtype);
+}
+
 // blackman_window_size (FourierProject.hpp:114-137).
 int blackman_window_size(float fftfreq_blackman, float spectrum_size) {
     double samples = static_cast<double>(spectrum_size) * static_cast<double>(fftfreq_blackman);
@@ -412,6 +425,7 @@ int prepare_extract(
     a.in_cplx = is_complex(volume->dtype);
     a.out_cplx = is_complex(slice->dtype);
     a.wide_in = needs_wide(volume) || needs_wide(volume_weight);
+    a.in_bytes_narrow = spans_bytes32(volume) && spans_bytes32(volume_weight);
     return NB_OK;
 }
 

@@ -238,8 +238,12 @@ batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_ite
             if constexpr (has_window<I>()) {
                 const int y = ty * VT.ty + ly;
                 const bool valid = u < R.a.slice_w / 2 + 1 && y < R.a.slice_h;
-                if (__any_sync(0xffffffffu, valid))
-                    extract_window_patch<I, IN_C, OUT_C, int>(R.a, b, y, u, valid, s_slots[warp], nullptr, 0);
+                if (__any_sync(0xffffffffu, valid)) {
+                    if (R.a.in_bytes_narrow)
+                        extract_window_patch<I, IN_C, OUT_C, uint32_t>(R.a, b, y, u, valid, s_slots[warp], nullptr, 0);
+                    else
+                        extract_window_patch<I, IN_C, OUT_C, int64_t>(R.a, b, y, u, valid, s_slots[warp], nullptr, 0);
+                }
             } else if (u < R.a.slice_w / 2 + 1) {
                 bool done = false;
                 if constexpr (I == I_LINEAR && IN_C) {

@@ -353,10 +353,10 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
         return a.wide_in ? launch_linear_volume<IN_C, OUT_C, int64_t>(a, stream)
                          : launch_linear_volume<IN_C, OUT_C, int32_t>(a, stream);
     if constexpr (has_window<I>()) {
-        if (a.wide_in)
-            extract_window_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+        if (a.in_bytes_narrow)
+            extract_window_kernel<I, IN_C, OUT_C, uint32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
         else
-            extract_window_kernel<I, IN_C, OUT_C, int32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
+            extract_window_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
     } else {
         if (a.wide_in)
             extract_kernel<I, IN_C, OUT_C, int64_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);

@@ -5,7 +5,7 @@
 // warp's load touches 32 unrelated places (19 sectors a request for LANCZOS8), each a pass of its own
 // through the L1. Here the lanes of a group (4 for SIZE 4, else 8) read one row of one pixel together,
 // consecutive in memory, so one request serves 4 pixels and touches their 4 rows: LANCZOS8, 500 slices of
-// 192^2, 5180 us -> 2286 us (2.27x).
+// 192^2, 5180 us -> 2200 us (2286 us without the simple cells' path below).
 //
 // A warp works in three phases. (1) One lane per pixel: coordinates, cutoff, and the pixel's cell and
 // three sets of tap weights into a shared slot; pixels outside the cutoff take none. (2) One group per
@@ -35,12 +35,30 @@ struct WindowSlots {
 template<int I>
 constexpr bool has_window() { return InterpTraits<I>::SIZE >= 4; }
 
+// Adds up the lanes of each group; the first of them stores the value of slot `at`.
+template<typename S, bool CPLX>
+__device__ __forceinline__ void group_sum(S& s, float2 sum, int j, int at, int n) {
+#pragma unroll
+    for (int o = S::LANES / 2; o > 0; o /= 2) {
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+        if constexpr (CPLX)
+            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+    }
+    if (j == 0 && at < n)
+        s.value[at] = sum;
+}
+
+// Whether the taps b + [0, size) along an axis of n frequencies all exist and follow each other in memory.
+__device__ __forceinline__ bool simple_axis(bool centered, int b, int size, int n) {
+    return b >= -n / 2 && b <= (n - 1) / 2 - (size - 1) && (centered || b >= 0 || b <= -size);
+}
+
 // Values of `n` slots' samples of the volume `v`, into s.value. All lanes of the warp call it together.
 template<int I, bool CPLX, typename Idx>
 __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectrum3& sp, WindowSlots<I>& s, int n) {
     using S = WindowSlots<I>;
     constexpr int SIZE = S::SIZE, LANES = S::LANES, START = -(SIZE - 1) / 2;
-    constexpr unsigned FULL = (1u << SIZE) - 1u;
+    using T = typename std::conditional<CPLX, float2, float>::type;
     const int lane = threadIdx.x & 31;
     const int j = lane % LANES;
     const int lo0 = -sp.n0 / 2, hi0 = (sp.n0 - 1) / 2;
@@ -55,6 +73,42 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
 #pragma unroll
         for (int k = 0; k < S::AXIS; k += 4)
             *reinterpret_cast<float4*>(w1 + k) = *reinterpret_cast<const float4*>(slot + 4 + S::AXIS + k);
+        float2 sum = make_float2(0.f, 0.f);
+        unsigned long long sum2 = 0, w12[SIZE];
+        if constexpr (CPLX) {
+#pragma unroll
+            for (int k = 0; k < SIZE; ++k)
+                w12[k] = pack2(w1[k], w1[k]);
+        }
+        if (CPLX && __all_sync(0xffffffffu, cell.w != 0.f)) {
+            // Simple cells: one offset per pixel, rows and planes at the volume's strides from it. With 32-bit
+            // byte offsets from the volume's base (Idx = uint32_t) a row costs one addition.
+            const T* from = static_cast<const T*>(v.data);
+            const Idx start = static_cast<Idx>(frequency2index(sp.centered, b0, sp.n0)) * v.s0 +
+                              static_cast<Idx>(frequency2index(sp.centered, b1, sp.n1)) * v.s1 +
+                              static_cast<Idx>(j < SIZE ? x : x - j) * v.s2;  // lanes past the window: its first column
+            Idx plane = start * static_cast<Idx>(sizeof(T));
+            const Idx to_plane = v.s0 * static_cast<Idx>(sizeof(T)), to_row = v.s1 * static_cast<Idx>(sizeof(T));
+#pragma unroll 1
+            for (int k0 = 0; k0 < SIZE; ++k0) {
+                unsigned long long e[SIZE], az = 0;
+                Idx row = plane;
+#pragma unroll
+                for (int k = 0; k < SIZE; ++k) {
+                    e[k] = __ldg(reinterpret_cast<const unsigned long long*>(reinterpret_cast<const char*>(from) + row));
+                    row += to_row;
+                }
+                const float w0 = slot[4 + k0];
+#pragma unroll
+                for (int k = 0; k < SIZE; ++k)
+                    az = fma2(e[k], w12[k], az);
+                sum2 = fma2(az, pack2(w0, w0), sum2);
+                plane += to_plane;
+            }
+            sum = j < SIZE ? cmul(unpack2(sum2), slot[4 + 2 * S::AXIS + j]) : make_float2(0.f, 0.f);
+            group_sum<S, CPLX>(s, sum, j, at, n);
+            continue;
+        }
         const bool mirror = x < 0;
         const int ix = mirror ? -x : x;
         const bool okx = j < SIZE && ix <= sp.n2 / 2;
@@ -69,18 +123,7 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
             okz |= z >= lo0 && z <= hi0 ? 1u << k : 0u;
             oy[k] = good ? static_cast<Idx>(frequency2index(sp.centered, y, sp.n1)) * v.s1 : 0;
         }
-        using T = typename std::conditional<CPLX, float2, float>::type;
         const T* column = static_cast<const T*>(v.data) + (okx ? static_cast<Idx>(ix) * v.s2 : 0);
-        float2 sum = make_float2(0.f, 0.f);
-        unsigned long long sum2 = 0, w12[SIZE];
-        if constexpr (CPLX) {
-#pragma unroll
-            for (int k = 0; k < SIZE; ++k)
-                w12[k] = pack2(w1[k], w1[k]);
-        }
-        // Interior cells: every tap of every lane is in the volume (an x tap that is not, or a lane without
-        // one, reads the column x = 0 and is left out of the sum below).
-        const bool interior = __all_sync(0xffffffffu, oky == FULL && okz == FULL);
 #pragma unroll 1
         for (int k0 = 0; k0 < SIZE; ++k0) {
             const int z = mirror ? -(b0 + k0) : b0 + k0;
@@ -89,16 +132,10 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
             const T* row = column + (goodz ? static_cast<Idx>(frequency2index(sp.centered, z, sp.n0)) * v.s0 : 0);
             if constexpr (CPLX) {
                 unsigned long long e[SIZE], az = 0;
-                if (interior) {
 #pragma unroll
-                    for (int k = 0; k < SIZE; ++k)
-                        e[k] = __ldg(reinterpret_cast<const unsigned long long*>(row + oy[k]));
-                } else {
-#pragma unroll
-                    for (int k = 0; k < SIZE; ++k)
-                        e[k] = goodz && ((oky >> k) & 1u)
-                                   ? __ldg(reinterpret_cast<const unsigned long long*>(row + oy[k])) : 0ull;
-                }
+                for (int k = 0; k < SIZE; ++k)
+                    e[k] = goodz && ((oky >> k) & 1u)
+                               ? __ldg(reinterpret_cast<const unsigned long long*>(row + oy[k])) : 0ull;
 #pragma unroll
                 for (int k = 0; k < SIZE; ++k)
                     az = fma2(e[k], w12[k], az);
@@ -118,14 +155,7 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
         sum = okx ? cmul(sum, slot[4 + 2 * S::AXIS + j]) : make_float2(0.f, 0.f);
         if (mirror)
             sum.y = -sum.y;
-#pragma unroll
-        for (int o = LANES / 2; o > 0; o /= 2) {
-            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
-            if constexpr (CPLX)
-                sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
-        }
-        if (j == 0 && at < n)
-            s.value[at] = sum;
+        group_sum<S, CPLX>(s, sum, j, at, n);
     }
     __syncwarp();
 }
@@ -171,11 +201,15 @@ __device__ __forceinline__ void extract_window_patch(const ProjArgs& a, int64_t 
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const float fl = floorf(q[k]);
-                cell[k] = static_cast<int>(fl);
+                cell[k] = static_cast<int>(fminf(fmaxf(fl, -1e9f), 1e9f));  // far outside: no tap either way
                 interp_weights<I>(sub(q[k], fl), ws[k]);
             }
             float4* slot = reinterpret_cast<float4*>(s.slot[at]);
-            slot[0] = make_float4(__int_as_float(cell[0]), __int_as_float(cell[1]), __int_as_float(cell[2]), 0.f);
+            constexpr int START = -(S::SIZE - 1) / 2;
+            const bool simple = simple_axis(sp.centered, cell[0] + START, S::SIZE, sp.n0) &&
+                                simple_axis(sp.centered, cell[1] + START, S::SIZE, sp.n1) &&
+                                cell[2] >= -START && cell[2] <= sp.n2 / 2 - (S::SIZE - 1) - START;
+            slot[0] = make_float4(__int_as_float(cell[0]), __int_as_float(cell[1]), __int_as_float(cell[2]), simple ? 1.f : 0.f);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
 #pragma unroll

@@ -4,7 +4,8 @@
 
 Each .cu under noa_b200/csrc is compiled with nvcc for sm_100a (-gencode arch=compute_100a,code=sm_100a)
 in parallel, then linked into one shared library with the CUDA runtime linked statically, so it loads
-beside any PyTorch build. Rebuilds only what changed.
+beside any PyTorch build; noa_b200/_lib/_marshal.so is the Python API's native marshalling. Rebuilds only
+what changed.
 """
 from __future__ import annotations
 
@@ -14,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -64,9 +66,24 @@ def _compile(src: str, verbose_ptxas: bool) -> tuple[str, str]:
     return obj, r.stderr
 
 
+def _build_marshal() -> None:
+    """The Python API's native marshalling (csrc/marshal.c). Without Python's headers the API marshals
+    through ctypes instead."""
+    src, out = os.path.join(CSRC, "marshal.c"), os.path.join(LIBDIR, "_marshal.so")
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")) or not _stale(out, [src] + _headers()):
+        return
+    cmd = [shutil.which("gcc") or "cc", "-O2", "-fPIC", "-shared", "-Wall", "-Wextra", "-I", INCLUDE, "-I", include,
+           src, "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {src} failed:\n{r.stdout}\n{r.stderr}")
+
+
 def build(verbose_ptxas: bool = False, jobs: int | None = None) -> str:
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(LIBDIR, exist_ok=True)
+    _build_marshal()
     srcs = _sources()
     with cf.ThreadPoolExecutor(max_workers=jobs or min(8, os.cpu_count() or 1)) as ex:
         results = list(ex.map(lambda s: _compile(s, verbose_ptxas), srcs))

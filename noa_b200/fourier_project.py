@@ -11,6 +11,8 @@ There is no CPU fallback: if the CUDA library is missing, importing the function
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 from dataclasses import dataclass
 
@@ -104,19 +106,28 @@ def library_path() -> str:
 # ---------------------------------------------------------------------------------------------------
 # Argument marshalling.
 # ---------------------------------------------------------------------------------------------------
+_TORCH: list = []
+
+
 def _torch():
-    import torch
-    return torch
+    if not _TORCH:
+        import torch
+        _TORCH.append(torch)
+    return _TORCH[0]
 
 
 _DTYPES: dict = {}
 
 
-def _dtype_code(t) -> int:
+def _fill_dtypes() -> None:
     if not _DTYPES:
         torch = _torch()
         _DTYPES.update({torch.float32: DTYPE_F32, torch.complex64: DTYPE_C32,
                         torch.float64: DTYPE_F64, torch.complex128: DTYPE_C64})
+
+
+def _dtype_code(t) -> int:
+    _fill_dtypes()
     return _DTYPES[t.dtype]
 
 
@@ -240,6 +251,8 @@ def _options(interp="linear", fftfreq_cutoff=0.5, target_shape=None, ews_radius=
 def _stream_ptr(stream) -> int | None:
     torch = _torch()
     if stream is None:
+        if torch.cuda.is_initialized():  # current_stream() without making its object
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
@@ -263,19 +276,67 @@ def _ref(x):
 
 
 # ---------------------------------------------------------------------------------------------------
+# Calls: natively (csrc/marshal.c, built beside the library), or through the ctypes structures where that
+# module was not built (no Python headers). Both fill the same structures from the same arguments.
+# ---------------------------------------------------------------------------------------------------
+_MARSHAL_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_marshal.so")
+_native_module: list = []
+_ADDRESSES: dict = {}
+
+
+def _native():
+    """The marshalling module, or None if it was not built."""
+    if not _native_module:
+        module = None
+        if os.path.exists(_MARSHAL_PATH):
+            loader = importlib.machinery.ExtensionFileLoader("_marshal", _MARSHAL_PATH)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_marshal", loader))
+            loader.exec_module(module)
+            torch = _torch()
+            _fill_dtypes()
+            module.init(NoaB200Error, _DTYPES, INTERPS, as_nb_transform, torch.float32, torch.Tensor)
+        _native_module.append(module)
+    return _native_module[0]
+
+
+def _address(name: str) -> int:
+    a = _ADDRESSES.get(name)
+    if a is None:
+        a = _ADDRESSES[name] = C.cast(getattr(lib(), name), C.c_void_p).value
+    return a
+
+
+def _call(name, remap, input, input_weight, input_shape, output, output_weight, output_shape, transforms, options,
+          stream) -> None:
+    """One call of the entry point `name`. `transforms`: scaling, rotation, of one or both sides; `options`:
+    (interp, fftfreq_cutoff, target_shape, ews_radius, windowed_sinc, w_windowed_sinc, add_to_output,
+    correct_weights)."""
+    native = _native()
+    if native is not None:
+        code = native.call(_address(name), REMAPS[remap], input, input_weight, input_shape, output, output_weight,
+                           output_shape, options, _stream_ptr(stream), *transforms)
+    else:
+        keep = []
+        o = _options(*options)
+        code = getattr(lib(), name)(
+            REMAPS[remap], _ref(as_nb_array(input, keep)), _ref(as_nb_array(input_weight, keep)),
+            _shape(input_shape), _ref(as_nb_array(output, keep)), _ref(as_nb_array(output_weight, keep)),
+            _shape(output_shape), *[_ref(as_nb_transform(x, k % 2 == 1, keep)) for k, x in enumerate(transforms)],
+            C.byref(o), _stream_ptr(stream))
+    if code != NB_OK:
+        _check(code)
+
+
+# ---------------------------------------------------------------------------------------------------
 # noa::xform API.
 # ---------------------------------------------------------------------------------------------------
 def rasterize_central_slices_3d(remap: str, slice, slice_weight, slice_shape, volume, volume_weight,
                                 volume_shape, inv_scaling, fwd_rotation, *, fftfreq_cutoff=0.5,
                                 target_shape=None, ews_radius=(0.0, 0.0), stream=None) -> None:
     """noa::xform::rasterize_central_slices_3d (FourierProject.hpp:1653-1692): trilinear insertion (+=)."""
-    keep = []
-    o = _options(fftfreq_cutoff=fftfreq_cutoff, target_shape=target_shape, ews_radius=ews_radius)
-    _check(lib().nb_rasterize_central_slices_3d(
-        REMAPS[remap], _ref(as_nb_array(slice, keep)), _ref(as_nb_array(slice_weight, keep)), _shape(slice_shape),
-        _ref(as_nb_array(volume, keep)), _ref(as_nb_array(volume_weight, keep)), _shape(volume_shape),
-        _ref(as_nb_transform(inv_scaling, False, keep)), _ref(as_nb_transform(fwd_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = ("linear", fftfreq_cutoff, target_shape, ews_radius, None, None, False, False)
+    _call("nb_rasterize_central_slices_3d", remap, slice, slice_weight, slice_shape, volume, volume_weight,
+          volume_shape, (inv_scaling, fwd_rotation), o, stream)
 
 
 def rasterize_central_slices_3d_static_scratch(remap: str, slice, slice_weight, slice_shape, volume, volume_weight,
@@ -287,27 +348,18 @@ def rasterize_central_slices_3d_static_scratch(remap: str, slice, slice_weight, 
     64 MiB array reserved per GPU when the library loads: with weights, volumes up to 4,194,304 rfft
     voxels (complex) are accepted, larger ones raise. Calls share that array, so calls that overlap on
     the GPU must be ordered; the first call on a device should come before any stream capture."""
-    keep = []
-    o = _options(fftfreq_cutoff=fftfreq_cutoff, target_shape=target_shape, ews_radius=ews_radius)
-    _check(lib().nb_rasterize_central_slices_3d_static_scratch(
-        REMAPS[remap], _ref(as_nb_array(slice, keep)), _ref(as_nb_array(slice_weight, keep)), _shape(slice_shape),
-        _ref(as_nb_array(volume, keep)), _ref(as_nb_array(volume_weight, keep)), _shape(volume_shape),
-        _ref(as_nb_transform(inv_scaling, False, keep)), _ref(as_nb_transform(fwd_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = ("linear", fftfreq_cutoff, target_shape, ews_radius, None, None, False, False)
+    _call("nb_rasterize_central_slices_3d_static_scratch", remap, slice, slice_weight, slice_shape, volume,
+          volume_weight, volume_shape, (inv_scaling, fwd_rotation), o, stream)
 
 
 def insert_central_slices_3d(remap: str, slice, slice_weight, slice_shape, volume, volume_weight, volume_shape,
                              fwd_scaling, inv_rotation, *, interp="linear", windowed_sinc=None,
                              fftfreq_cutoff=0.5, target_shape=None, ews_radius=(0.0, 0.0), stream=None) -> None:
     """noa::xform::insert_central_slices_3d (FourierProject.hpp:1770-1815): windowed-sinc gather (+=)."""
-    keep = []
-    o = _options(interp=interp, fftfreq_cutoff=fftfreq_cutoff, target_shape=target_shape,
-                 ews_radius=ews_radius, windowed_sinc=windowed_sinc)
-    _check(lib().nb_insert_central_slices_3d(
-        REMAPS[remap], _ref(as_nb_array(slice, keep)), _ref(as_nb_array(slice_weight, keep)), _shape(slice_shape),
-        _ref(as_nb_array(volume, keep)), _ref(as_nb_array(volume_weight, keep)), _shape(volume_shape),
-        _ref(as_nb_transform(fwd_scaling, False, keep)), _ref(as_nb_transform(inv_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = (interp, fftfreq_cutoff, target_shape, ews_radius, windowed_sinc, None, False, False)
+    _call("nb_insert_central_slices_3d", remap, slice, slice_weight, slice_shape, volume, volume_weight,
+          volume_shape, (fwd_scaling, inv_rotation), o, stream)
 
 
 def insert_central_slices_3d_scatter(remap: str, slice, slice_weight, slice_shape, volume, volume_weight,
@@ -316,14 +368,9 @@ def insert_central_slices_3d_scatter(remap: str, slice, slice_weight, slice_shap
                                      ews_radius=(0.0, 0.0), stream=None) -> None:
     """Slice-major atomic scatter form of ``insert_central_slices_3d``: the same terms, summed over the
     slices in an unspecified order (no counterpart in the reference; see fourier_project.h)."""
-    keep = []
-    o = _options(interp=interp, fftfreq_cutoff=fftfreq_cutoff, target_shape=target_shape,
-                 ews_radius=ews_radius, windowed_sinc=windowed_sinc)
-    _check(lib().nb_insert_central_slices_3d_scatter(
-        REMAPS[remap], _ref(as_nb_array(slice, keep)), _ref(as_nb_array(slice_weight, keep)), _shape(slice_shape),
-        _ref(as_nb_array(volume, keep)), _ref(as_nb_array(volume_weight, keep)), _shape(volume_shape),
-        _ref(as_nb_transform(fwd_scaling, False, keep)), _ref(as_nb_transform(inv_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = (interp, fftfreq_cutoff, target_shape, ews_radius, windowed_sinc, None, False, False)
+    _call("nb_insert_central_slices_3d_scatter", remap, slice, slice_weight, slice_shape, volume, volume_weight,
+          volume_shape, (fwd_scaling, inv_rotation), o, stream)
 
 
 def fourier_interpolation_correction(input, output, interp="linear", post_correction=True, *, stream=None) -> None:
@@ -341,14 +388,9 @@ def extract_central_slices_3d(remap: str, volume, volume_weight, volume_shape, s
                               inv_scaling, fwd_rotation, *, interp="linear", w_windowed_sinc=None,
                               fftfreq_cutoff=0.5, target_shape=None, ews_radius=(0.0, 0.0), stream=None) -> None:
     """noa::xform::extract_central_slices_3d (FourierProject.hpp:1869-1914)."""
-    keep = []
-    o = _options(interp=interp, fftfreq_cutoff=fftfreq_cutoff, target_shape=target_shape,
-                 ews_radius=ews_radius, w_windowed_sinc=w_windowed_sinc)
-    _check(lib().nb_extract_central_slices_3d(
-        REMAPS[remap], _ref(as_nb_array(volume, keep)), _ref(as_nb_array(volume_weight, keep)), _shape(volume_shape),
-        _ref(as_nb_array(slice, keep)), _ref(as_nb_array(slice_weight, keep)), _shape(slice_shape),
-        _ref(as_nb_transform(inv_scaling, False, keep)), _ref(as_nb_transform(fwd_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = (interp, fftfreq_cutoff, target_shape, ews_radius, None, w_windowed_sinc, False, False)
+    _call("nb_extract_central_slices_3d", remap, volume, volume_weight, volume_shape, slice, slice_weight,
+          slice_shape, (inv_scaling, fwd_rotation), o, stream)
 
 
 def insert_and_extract_central_slices_3d(remap: str, input_slice, input_weight, input_slice_shape, output_slice,
@@ -358,17 +400,11 @@ def insert_and_extract_central_slices_3d(remap: str, input_slice, input_weight, 
                                          correct_weights=False, fftfreq_cutoff=0.5, ews_radius=(0.0, 0.0),
                                          stream=None) -> None:
     """noa::xform::insert_and_extract_central_slices_3d (FourierProject.hpp:1987-2049)."""
-    keep = []
-    o = _options(interp=interp, fftfreq_cutoff=fftfreq_cutoff, ews_radius=ews_radius,
-                 windowed_sinc=input_windowed_sinc, w_windowed_sinc=w_windowed_sinc,
-                 add_to_output=add_to_output, correct_weights=correct_weights)
-    _check(lib().nb_insert_and_extract_central_slices_3d(
-        REMAPS[remap], _ref(as_nb_array(input_slice, keep)), _ref(as_nb_array(input_weight, keep)),
-        _shape(input_slice_shape),
-        _ref(as_nb_array(output_slice, keep)), _ref(as_nb_array(output_weight, keep)), _shape(output_slice_shape),
-        _ref(as_nb_transform(input_fwd_scaling, False, keep)), _ref(as_nb_transform(input_inv_rotation, True, keep)),
-        _ref(as_nb_transform(output_inv_scaling, False, keep)), _ref(as_nb_transform(output_fwd_rotation, True, keep)),
-        C.byref(o), _stream_ptr(stream)))
+    o = (interp, fftfreq_cutoff, None, ews_radius, input_windowed_sinc, w_windowed_sinc, add_to_output,
+         correct_weights)
+    _call("nb_insert_and_extract_central_slices_3d", remap, input_slice, input_weight, input_slice_shape,
+          output_slice, output_weight, output_slice_shape,
+          (input_fwd_scaling, input_inv_rotation, output_inv_scaling, output_fwd_rotation), o, stream)
 
 
 def version() -> str:

@@ -1,0 +1,91 @@
+"""The native marshalling fills the structures that the ctypes path fills, and refuses what it refuses (CPU)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from noa_b200 import fourier_project as fp
+
+pytestmark = pytest.mark.skipif(fp._native() is None, reason="built without Python headers")
+
+_P = C.c_void_p
+_ENTRY = {n: C.CFUNCTYPE(C.c_int, C.c_int32, *([_P] * (8 + n))) for n in (2, 4)}
+
+
+def _bytes(address, struct):
+    return None if not address else C.string_at(address, C.sizeof(struct))
+
+
+def _seen(monkeypatch, native, call, n_transforms):
+    """What the entry point gets from `call`, by value."""
+    got = []
+
+    def entry(remap, *p):
+        got.append((remap, [_bytes(p[i], fp.NbArray) for i in (0, 1, 3, 4)],
+                    [_bytes(p[i], C.c_int64 * 4) for i in (2, 5)],
+                    [_bytes(p[6 + i], fp.NbTransform) for i in range(n_transforms)],
+                    _bytes(p[6 + n_transforms], fp.NbOptions), p[7 + n_transforms]))
+        return 0
+
+    function = _ENTRY[n_transforms](entry)
+    with monkeypatch.context() as m:
+        if native:
+            m.setattr(fp, "_address", lambda name: C.cast(function, _P).value)
+        else:
+            m.setattr(fp, "_native", lambda: None)
+            m.setattr(fp, "lib", lambda: type("Lib", (), {"__getattr__": lambda self, name: function}, )())
+            m.setattr(fp, "_default_options", lambda: fp.NbOptions(interp=1))
+        call()
+    return got
+
+
+_vol = torch.zeros((1, 8, 8, 5), dtype=torch.complex64)
+_out = torch.zeros((3, 1, 8, 9), dtype=torch.float32)[..., ::2]
+_w = torch.zeros((3, 1, 8, 5))
+_rot, _quat, _scale = torch.eye(3).repeat(3, 1, 1), torch.zeros((3, 4)), torch.zeros((3, 2, 2))
+_packed = fp.pack_rotations(_rot)
+
+
+@pytest.mark.parametrize("volume", [_vol, 2.5, 3, 1 + 2j, np.float64(4.0)], ids=str)
+@pytest.mark.parametrize("weight", [_w, None])
+@pytest.mark.parametrize("rotation", [_packed, _quat, np.eye(3), (0, 0, 0, 1)], ids=["mat33", "quat", "one", "inline"])
+@pytest.mark.parametrize("kw", [{}, dict(interp="lanczos8", fftfreq_cutoff=1, ews_radius=3.5, target_shape=[1, 9, 9, 9, 7]),
+                                dict(interp=101, w_windowed_sinc=fp.WindowedSinc(0.1, 1), ews_radius=np.array([1.0, 2.0]))],
+                         ids=["default", "options", "more"])
+def test_same_structures(monkeypatch, volume, weight, rotation, kw):
+    for scaling in (None, _scale, np.eye(2)):
+        def call():
+            fp.extract_central_slices_3d("hc2h", volume, None, (1, 8, 8, 8), _out, weight, torch.Size((3, 1, 8, 8)), scaling,
+                                         rotation, stream=77, **kw)
+        a, b = _seen(monkeypatch, True, call, 2), _seen(monkeypatch, False, call, 2)
+        assert a == b and len(a) == 1
+
+
+def test_same_structures_of_both_sides(monkeypatch):
+    def call():
+        fp.insert_and_extract_central_slices_3d(
+            "h2h", _w, 2.0, (3, 1, 8, 8), _out, _w, np.array([3, 1, 8, 8]), _scale, _packed, None, _quat,
+            input_windowed_sinc=fp.WindowedSinc(0.2, 0.3), add_to_output=np.bool_(True), correct_weights=0, stream=5)
+    a, b = _seen(monkeypatch, True, call, 4), _seen(monkeypatch, False, call, 4)
+    assert a == b and len(a) == 1
+
+
+@pytest.mark.parametrize("change", [dict(volume=_vol[0]), dict(volume=torch.zeros((1, 8, 8, 5), dtype=torch.int32)),
+                                    dict(rotation=None), dict(rotation=np.zeros((2, 3))), dict(rotation=_quat.double()),
+                                    dict(rotation=torch.zeros((3, 5))), dict(shape=(1, 8, 8, 8, 8)), dict(interp="none"),
+                                    dict(target_shape=(1, 2)), dict(volume="x"), dict(remap="h2x"), dict(interp=None)],
+                         ids=str)
+def test_same_refusals(monkeypatch, change):
+    a = dict(volume=_vol, rotation=_packed, shape=(1, 8, 8, 8), interp="linear", target_shape=None, remap="hc2h")
+    a.update(change)
+
+    def call():
+        fp.extract_central_slices_3d(a["remap"], a["volume"], None, a["shape"], _out, None, (3, 1, 8, 8), None, a["rotation"],
+                                     interp=a["interp"], target_shape=a["target_shape"], stream=0)
+    errors = []
+    for native in (True, False):
+        with pytest.raises(Exception) as e:
+            _seen(monkeypatch, native, call, 2)
+        errors.append((type(e.value), getattr(e.value, "code", None)))
+    assert errors[0] == errors[1]

@@ -55,12 +55,11 @@ enum { NB_BATCH_AUTOTUNE = 1, NB_BATCH_PERSISTENT_ONLY = 2 };
  * in the text file $NB_AUTOTUNE_CACHE or $HOME/.cache/noa_b200/autotune.txt; autotuning runs the batch,
  * so it writes the outputs) and captures the launch into a CUDA graph. Synchronizes `stream`.
  * LINEAR batches over complex volumes (no scaling, EWS, input weights or w-window) hold a pair copy
- * (16 bytes per rfft voxel) of each volume whose requests read at least twice as many pixels as it
- * has voxels, like the per-call entry point; the graph rebuilds these copies at every run, so changes
- * to the volumes between runs are seen. A request read through a pair copy with at least 2^23 output
- * pixels runs, in the graph, as a grid of its own (the per-call pair kernel) on a parallel branch that
- * starts when its volume's copy is written; the copies of the other volumes are made meanwhile on a
- * higher-priority branch (NB_BATCH_PERSISTENT_ONLY keeps every request in the persistent kernel).
+ * (16 bytes per rfft voxel) of each volume whose requests read enough pixels to pay for it (at least
+ * three per voxel), like the per-call entry point; the graph rebuilds these copies at every run, so
+ * changes to the volumes between runs are seen. A LINEAR request with at least 2^16 output pixels runs,
+ * in the graph, as a grid of its own (the per-call kernel) on a parallel branch, from its volume or, once
+ * it is written, from its volume's copy; the copies are made meanwhile on a higher-priority branch (NB_BATCH_PERSISTENT_ONLY keeps every request in the persistent kernel).
  * Results are bit-identical either way. */
 NB_API int nb_extract_batch_create(int32_t remap, const nb_extract_request* requests, int64_t n_requests,
                                    const nb_options* options, int32_t flags, void* stream,
@@ -92,9 +91,8 @@ typedef struct {
 } nb_extract_request_ex;
 
 /* Validates the requests and enqueues them on `stream` (no graph, no autotuning: the configuration
- * cached for the workload key is used when there is one, else a default): each request read through
- * its pair copy with at least 2^21 output pixels as a grid of its own (the per-call pair kernel), the
- * others as ONE persistent launch, its descriptors staged in stream-ordered device memory. The request
+ * cached for the workload key is used when there is one, else a default): each LINEAR request
+ * with at least 2^21 output pixels as a grid of its own (the per-call kernel), the others as ONE persistent launch, its descriptors staged in stream-ordered device memory. The request
  * structs may be freed on return; the device buffers must stay valid until the launches complete.
  * Results are bit-identical to nb_extract_central_slices_3d on each request. */
 NB_API int nb_extract_batch_launch(int32_t remap, const nb_extract_request_ex* requests, int64_t n_requests,

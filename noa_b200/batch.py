@@ -163,7 +163,7 @@ def extract_batch_launch(remap: str, requests: list[ExtractRequest], pairs: list
                          interp="linear", fftfreq_cutoff=0.5, w_windowed_sinc=None, ews_radius=(0.0, 0.0),
                          persistent_only=False, stream=None) -> None:
     """Enqueues many extract_central_slices_3d calls on ``stream`` (no graph, no autotuning): requests
-    of at least 2^21 output pixels read through their pair copy as grids of their own, the others as
+    of at least 2^21 output pixels (LINEAR) as grids of their own, the others as
     ONE persistent launch (every request, with ``persistent_only``). ``pairs[i]`` is an optional
     ``volume_pairs`` copy of request i's volume."""
     lib = fp.lib()
@@ -186,8 +186,7 @@ def extract_batch_launch(remap: str, requests: list[ExtractRequest], pairs: list
 class ExtractBatch:
     """A captured batch of extractions. ``autotune=True`` times tile shapes and CTAs per SM on this
     batch (once per workload key; the choice is cached) before capturing the launch. LINEAR requests
-    of at least 2^23 output pixels read through a pair copy run as grids of their own inside the
-    graph, unless ``persistent_only=True``."""
+    of at least 2^16 output pixels run as grids of their own inside the graph, unless ``persistent_only=True``."""
 
     def __init__(self, remap: str, requests: list[ExtractRequest], *, interp="linear", fftfreq_cutoff=0.5,
                  w_windowed_sinc=None, ews_radius=(0.0, 0.0), autotune=True, persistent_only=False, stream=None):

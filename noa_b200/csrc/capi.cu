@@ -425,6 +425,7 @@ int prepare_extract(
     a.in_cplx = is_complex(volume->dtype);
     a.out_cplx = is_complex(slice->dtype);
     a.wide_in = needs_wide(volume) || needs_wide(volume_weight);
+    dense_pairs(a);
     a.in_bytes_narrow = spans_bytes32(volume) && spans_bytes32(volume_weight);
     return NB_OK;
 }
@@ -614,6 +615,7 @@ int nb_volume_pairs(const nb_array* volume, const int64_t volume_shape[4], void*
     a.in_cplx = 1;
     a.interp = I_LINEAR;
     a.wsize = 1;
+    dense_pairs(a);
     if (!pairs_apply(a))
         return fail(NB_ERROR_INVALID, "the pair copy must span fewer than 2^31 voxels");
     if ((st = check_pairs(pairs, pairs_bytes, a, "pairs")) != NB_OK)

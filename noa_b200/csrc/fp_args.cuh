@@ -39,6 +39,7 @@ struct ProjArgs {
 
     int in_cplx, out_cplx;     // value kinds (input/output complex?)
     int wide_in;               // input offsets need 64 bits (an array spans >= 2^31 elements)
+    int pair_sz, pair_sy;      // extract: element strides of the volume's pair copy (fp_pairs.cuh)
     int in_bytes_narrow;       // extract: byte offsets of the volume and its weights fit 32 bits unsigned
     int in_slice_narrow;       // offsets within one input slice fit 32 bits
 };

@@ -54,7 +54,7 @@ struct BatchReq {
 static_assert(sizeof(BatchReq) % 8 == 0, "BatchReq is staged in shared memory as 8-byte words");
 
 constexpr int PAIRS_PPT = 4;
-// Output pixels from which a request over a pair copy gets a grid of its own (about 8 slices of 128^2;
+// Output pixels from which a LINEAR request gets a grid of its own (about 8 slices of 128^2;
 // smaller requests go through the persistent kernel). Measured on 12,000 LINEAR slices over 12
 // volumes of 128-384 as 12, 120 and 600 requests: with grids of their own on 4 branches, 4.76, 4.61
 // and 4.70 ms against 5.36, 5.78 and 6.57 ms all in the persistent kernel (per-call 4.94, 7.57, 13.2).
@@ -71,12 +71,11 @@ template<bool OUT_C>
 __device__ __forceinline__ void extract_rows_pairs(const ProjArgs& a, const float4* pairs, int64_t b, int y0,
                                                    int dy, int u) {
     const Spectrum3 sp{a.vol_d, a.vol_h, a.vol_w, a.in_centered};
-    const int WP = a.vol_w / 2 + 1;
     const float f1 = div(static_cast<float>(u), a.f_slice1);
     float2 value[PAIRS_PPT];
     bool inside[PAIRS_PPT];
-    const float* m = nullptr;
-    const bool lean = lean_rotation(a, b, m);
+    LeanColumn column;
+    const bool lean = column.load(a, b, f1);
 #pragma unroll
     for (int r = 0; r < PAIRS_PPT; ++r) {
         const int y = y0 + r * dy;
@@ -87,12 +86,12 @@ __device__ __forceinline__ void extract_rows_pairs(const ProjArgs& a, const floa
         const float f0 = div(static_cast<float>(index2frequency(a.out_centered, y, a.slice_h)), a.f_slice0);
         float fz, fy, fx;
         if (lean)
-            slice2grid_lean(m, f0, f1, fz, fy, fx);
+            column.at(f0, fz, fy, fx);
         else
             slice2grid(f0, f1, a.scale, a.rot, b, a.ews, fz, fy, fx);
         inside[r] = dot3(fz, fy, fx, fz, fy, fx) <= a.cutoff_sqd;
         if (inside[r])
-            value[r] = to_output<true, OUT_C>(interp_linear_pairs(pairs, a.vol_h * WP, WP, sp, mul(fz, a.target0),
+            value[r] = to_output<true, OUT_C>(interp_linear_pairs(pairs, a.pair_sz, a.pair_sy, sp, mul(fz, a.target0),
                                                                   mul(fy, a.target1), mul(fx, a.target2)));
     }
 #pragma unroll
@@ -163,9 +162,9 @@ template<int I, bool WINDOW = has_window<I>()> struct BatchSlots { using T = Win
 template<int I> struct BatchSlots<I, false> { struct T {}; };
 
 // PAIRS_ONLY: every request reads a pair copy (LINEAR, complex); the generic path is compiled out so
-// the kernel fits 40 registers (6 CTAs per SM, like extract_pairs_kernel).
+// the kernel fits 48 registers (5 CTAs per SM, like extract_linear_kernel).
 template<int I, bool IN_C, bool OUT_C, int V, bool PAIRS_ONLY = false>
-__global__ void __launch_bounds__(256, PAIRS_ONLY ? 6 : VARIANTS[V].min_ctas)
+__global__ void __launch_bounds__(256, PAIRS_ONLY ? 5 : VARIANTS[V].min_ctas)
 batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_items,
                      unsigned long long* __restrict__ counter) {
     constexpr Variant VT = VARIANTS[V];
@@ -279,7 +278,7 @@ struct ReqPack { BatchReq r[PACK]; };
 static_assert(sizeof(ReqPack) + 64 <= 32764, "the descriptor pack must fit the kernel parameter space");
 
 template<bool OUT_C>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, 5)
 batch_pairs_param_kernel(const __grid_constant__ ReqPack pack, int n_req, int64_t n_items,
                          unsigned long long* __restrict__ counter) {
     constexpr Variant VT = VARIANTS[0];
@@ -439,6 +438,22 @@ struct Config {
 
 using namespace nb;
 
+namespace nb {
+namespace {
+constexpr size_t NO_JOB = ~size_t(0);  // of a direct request that reads its volume, not a pair copy
+
+// Whether a request gets a grid of its own: LINEAR without a w-window and at least `least` output pixels.
+bool runs_direct(const BatchReq& r, int64_t least) {
+    return r.a.interp == I_LINEAR && r.a.wsize <= 1 &&
+           r.a.n_slices * r.a.slice_h * static_cast<int64_t>(r.a.slice_w / 2 + 1) >= least;
+}
+
+cudaError_t launch_direct(const BatchReq& r, cudaStream_t s) {
+    return r.pairs ? launch_extract_pairs(r.a, r.pairs, s) : launch_extract_volume(r.a, s);
+}
+} // namespace
+} // namespace nb
+
 struct nb_extract_batch_t {
     int device = 0;
     int interp = 1;
@@ -458,15 +473,15 @@ struct nb_extract_batch_t {
     // (their make_pairs launches are part of the graph), so later changes to the volumes are seen.
     std::vector<std::pair<nb::ProjArgs, float4*>> pair_jobs;
     bool pairs_only = false;  // every request reads a pair copy: the pairs-only kernel
-    // Requests over a pair copy with at least DIRECT_MIN_PIXELS output pixels leave the persistent
-    // kernel: each runs the per-call pair kernel as a grid of its own on one of N_SIDE branches of the
-    // graph, as soon as its volume's copy is written, while the copies of the next volumes are made on
-    // a higher-priority branch. The per-call kernel's per-pixel cost is lower than the persistent
+    // Requests with at least DIRECT_MIN_PIXELS output pixels leave the persistent kernel: each runs the
+    // per-call kernel as a grid of its own on one of N_SIDE branches of the graph, from its volume where
+    // no pair copy is made, else as soon as that copy is written, while the copies of the next volumes are
+    // made on a higher-priority branch. The per-call kernel's per-pixel cost is lower than the persistent
     // kernel's (no claims, request lookups or per-item tile setup), and with several branches the
     // grids' ramps and tails overlap. (The copies, HBM-bound, overlap the extractions only a little:
     // 0.62 ms of copies for 12 volumes of 128-384 saved 0.08 ms against copying first.)
     std::vector<BatchReq> direct;
-    std::vector<size_t> direct_job;      // pair_jobs index of each direct request's copy
+    std::vector<size_t> direct_job;      // pair_jobs index of each direct request's copy, or NO_JOB
     int64_t n_requests = 0;              // persistent + direct
     cudaStream_t copy_stream = nullptr, side[N_SIDE] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[N_SIDE + 1] = {};
@@ -590,9 +605,10 @@ cudaError_t launch(nb_extract_batch_t* h, const Config& c, cudaStream_t stream) 
     }
     for (size_t k = 0; k < h->direct.size(); ++k) {
         const cudaStream_t s = h->side[k % N_SIDE];
-        if ((err = cudaStreamWaitEvent(s, h->ev_pairs[h->direct_job[k]], 0)) != cudaSuccess)
+        if (h->direct_job[k] != NO_JOB &&
+            (err = cudaStreamWaitEvent(s, h->ev_pairs[h->direct_job[k]], 0)) != cudaSuccess)
             return err;
-        if ((err = launch_extract_pairs(h->direct[k].a, h->direct[k].pairs, s)) != cudaSuccess)
+        if ((err = launch_direct(h->direct[k], s)) != cudaSuccess)
             return err;
     }
     if ((err = launch_persistent(h, c, h->copy_stream)) != cudaSuccess)
@@ -636,11 +652,11 @@ double time_config(nb_extract_batch_t* h, const Config& c, cudaStream_t stream, 
     return result;
 }
 
-// LINEAR over complex volumes: a pair copy per distinct volume whose requests read at least twice
-// as many pixels as it has voxels (the per-call rule), allocated for the batch's lifetime. Without
-// memory for a copy, its requests take the generic path.
+// LINEAR batches: a pair copy per distinct complex volume whose requests read enough pixels to pay for
+// it (pairs_pay), allocated for the batch's lifetime; without one, or without memory for it, requests
+// read the volume. Then the requests that get grids of their own leave the list.
 void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
-    if (h->interp != I_LINEAR || !h->in_cplx)
+    if (h->interp != I_LINEAR)
         return;
     struct Vol { const ProjArgs* a; int64_t pixels; std::vector<size_t> reqs; };
     std::vector<Vol> vols;
@@ -663,14 +679,19 @@ void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
     }
     for (const Vol& v : vols) {
         const int64_t vox = static_cast<int64_t>(v.a->vol_d) * v.a->vol_h * (v.a->vol_w / 2 + 1);
-        if (v.pixels < 2 * vox)
+        if (!pairs_pay(v.pixels, vox))
             continue;
-        float4* buf = static_cast<float4*>(device_alloc(static_cast<size_t>(vox) * sizeof(float4)));
+        ProjArgs copy = *v.a;
+        pad_pairs(copy);
+        float4* buf = static_cast<float4*>(device_alloc(static_cast<size_t>(pair_elements(copy)) * sizeof(float4)));
         if (!buf)
             continue;  // no memory for the copy: these requests read the volume itself
-        h->pair_jobs.push_back({*v.a, buf});
-        for (size_t i : v.reqs)
+        h->pair_jobs.push_back({copy, buf});
+        for (size_t i : v.reqs) {
             h->host_reqs[i].pairs = buf;
+            h->host_reqs[i].a.pair_sz = copy.pair_sz;
+            h->host_reqs[i].a.pair_sy = copy.pair_sy;
+        }
     }
     // Copies in increasing size, so the first direct grids start early and the largest copies overlap
     // the extractions.
@@ -678,17 +699,17 @@ void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
         return static_cast<int64_t>(x.first.vol_d) * x.first.vol_h * x.first.vol_w <
                static_cast<int64_t>(y.first.vol_d) * y.first.vol_h * y.first.vol_w;
     });
+    // Requests that read their volume itself need no copy and come first, then those of each copy in turn.
     std::vector<BatchReq> keep;
-    for (size_t j = 0; j < h->pair_jobs.size(); ++j)
-        for (const BatchReq& r : h->host_reqs)
-            if (allow_direct && r.pairs == h->pair_jobs[j].second &&
-                r.a.n_slices * r.a.slice_h * static_cast<int64_t>(r.a.slice_w / 2 + 1) >= DIRECT_MIN_PIXELS) {
-                h->direct.push_back(r);
-                h->direct_job.push_back(j);
-            }
+    if (allow_direct)
+        for (size_t j = 0; j <= h->pair_jobs.size(); ++j)
+            for (const BatchReq& r : h->host_reqs)
+                if (runs_direct(r, DIRECT_MIN_PIXELS) && r.pairs == (j ? h->pair_jobs[j - 1].second : nullptr)) {
+                    h->direct.push_back(r);
+                    h->direct_job.push_back(j ? j - 1 : NO_JOB);
+                }
     for (const BatchReq& r : h->host_reqs)
-        if (!(allow_direct && r.pairs &&
-              r.a.n_slices * r.a.slice_h * static_cast<int64_t>(r.a.slice_w / 2 + 1) >= DIRECT_MIN_PIXELS))
+        if (!(allow_direct && runs_direct(r, DIRECT_MIN_PIXELS)))
             keep.push_back(r);
     h->host_reqs.swap(keep);
     bool all = true;
@@ -986,9 +1007,8 @@ int nb_extract_batch_launch_ex(int32_t remap, const nb_extract_request_ex* reque
     if (!(flags & NB_BATCH_PERSISTENT_ONLY)) {
         std::vector<BatchReq> keep;
         for (const BatchReq& r : h.host_reqs) {
-            if (r.pairs &&
-                r.a.n_slices * r.a.slice_h * static_cast<int64_t>(r.a.slice_w / 2 + 1) >= ONESHOT_DIRECT_MIN_PIXELS) {
-                const cudaError_t err = launch_extract_pairs(r.a, r.pairs, s);
+            if (runs_direct(r, ONESHOT_DIRECT_MIN_PIXELS)) {
+                const cudaError_t err = launch_direct(r, s);
                 if (err != cudaSuccess)
                     return finish_launch(err);
             } else {

@@ -60,7 +60,7 @@ __global__ void make_pairs(const __grid_constant__ ProjArgs a, float4* __restric
         const int64_t off = z * a.in.s0 + y * a.in.s1 + x * a.in.s2;
         const float2 v0 = vol[off];
         const float2 v1 = x + 1 < WP ? vol[off + a.in.s2] : make_float2(0.f, 0.f);
-        pairs[i] = make_float4(v0.x, v0.y, v1.x, v1.y);
+        pairs[z * static_cast<Idx>(a.pair_sz) + y * static_cast<Idx>(a.pair_sy) + x] = make_float4(v0.x, v0.y, v1.x, v1.y);
     }
 }
 
@@ -69,20 +69,23 @@ __global__ void make_pairs(const __grid_constant__ ProjArgs a, float4* __restric
 // (its 2-D frequency, its offset) is computed once for all slices, and what depends on the slice and the
 // column once for PPT pixels. PAIRS: the taps come from a pair copy (four 16-byte loads per pixel), else
 // from the volume (eight loads). Same bits
-// as one slice per CTA and one pixel at a time: 4096 slices of 256^3 1195 us -> 1164 us with the copy;
-// 150 slices of 200^3 without it 50.1 us -> 42.6 us.
+// as one slice per CTA and one pixel at a time: 4096 slices of 256^3 1195 us -> 1164 us with the copy
+// (1104 us with the copy padded, pad_pairs); 150 slices of 200^3 without it 50.1 us -> 41.2 us.
 template<bool PAIRS, bool IN_C, bool OUT_C, int PPT, typename Idx>
-__global__ void __launch_bounds__(EXTRACT_THREADS, PAIRS || PPT == 1 ? 5 : 4)
-extract_linear_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx, int per_cta) {
+__global__ void __launch_bounds__(EXTRACT_THREADS, 5)
+extract_linear_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx, int per_cta,
+                      bool lanes_16) {
     const int wp = a.slice_w / 2 + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y0 = (blockIdx.x / ntx) * (TY * PPT) + (warp >> 1) * 4 + (lane >> 3);
-    const int u = (blockIdx.x % ntx) * TX + (warp & 1) * 8 + (lane & 7);
+    // A warp's pixels: 4 x 8, 2 x 4 per eight lanes, over a pair copy; else 4 x 8, or 2 x 16 (lanes_16).
+    const int row = PAIRS ? (warp >> 1) * 4 + pair_row(lane) : lanes_16 ? warp * 2 + (lane >> 4) : (warp >> 1) * 4 + (lane >> 3);
+    const int column = PAIRS ? (warp & 1) * 8 + pair_column(lane) : lanes_16 ? lane & 15 : (warp & 1) * 8 + (lane & 7);
+    const int y0 = (blockIdx.x / ntx) * (TY * PPT) + row;
+    const int u = (blockIdx.x % ntx) * TX + column;
     if (u >= wp || y0 >= a.slice_h)
         return;
     const Spectrum3 sp{a.vol_d, a.vol_h, a.vol_w, a.in_centered};
-    const int WP = a.vol_w / 2 + 1;
-    const int sz = a.vol_h * WP, sy = WP;
+    const int sz = a.pair_sz, sy = a.pair_sy;
     const View3<Idx> vol{a.in.data, static_cast<Idx>(a.in.s0), static_cast<Idx>(a.in.s1), static_cast<Idx>(a.in.s2)};
     const bool has_out_w = a.out_w.present;
     const bool has_in_w = !PAIRS && a.in_w.present;
@@ -97,8 +100,8 @@ extract_linear_kernel(const __grid_constant__ ProjArgs a, const float4* __restri
          first += static_cast<int64_t>(gridDim.y) * per_cta) {
         const int64_t end = first + per_cta < a.n_slices ? first + per_cta : a.n_slices;
         for (int64_t b = first; b < end; ++b) {
-            const float* m = nullptr;
-            const bool lean = lean_rotation(a, b, m);
+            LeanColumn column_of;
+            const bool lean = column_of.load(a, b, f1);
             using T = typename std::conditional<OUT_C, float2, float>::type;
             T* out = static_cast<T*>(a.out.data) + (b * a.out.s0 + pixel);
             float* out_w = static_cast<float*>(a.out_w.data) + (b * a.out_w.s0 + pixel_w);
@@ -108,7 +111,7 @@ extract_linear_kernel(const __grid_constant__ ProjArgs a, const float4* __restri
                     break;
                 float fz, fy, fx;
                 if (lean)
-                    slice2grid_lean(m, f0[r], f1, fz, fy, fx);
+                    column_of.at(f0[r], fz, fy, fx);
                 else
                     slice2grid(f0[r], f1, a.scale, a.rot, b, a.ews, fz, fy, fx);
                 float2 value = make_float2(0.f, 0.f);
@@ -154,7 +157,11 @@ cudaError_t launch_linear(const ProjArgs& a, const float4* pairs, cudaStream_t s
     const int per_cta = slices_per_cta(static_cast<int64_t>(ntx) * nty, a.n_slices);
     const int64_t groups = (a.n_slices + per_cta - 1) / per_cta;
     const dim3 grid(static_cast<unsigned>(ntx * nty), static_cast<unsigned>(groups < 65535 ? groups : 65535));
-    extract_linear_kernel<PAIRS, IN_C, OUT_C, PPT, Idx><<<grid, EXTRACT_THREADS, 0, stream>>>(a, pairs, ntx, per_cta);
+    // Without a pair copy sixteen lanes share a pass of the L1, over 16 bank groups of 8 bytes. Planes that
+    // all start on the same banks (boxes that are a multiple of 32) are read with 3.4 lines a group by lanes
+    // in a row and 4.1 by lanes in two rows of 8, others with 2.5 and 2.3 (replayed on the CPU).
+    const bool lanes_16 = !PAIRS && a.in.s0 % 16 == 0;
+    extract_linear_kernel<PAIRS, IN_C, OUT_C, PPT, Idx><<<grid, EXTRACT_THREADS, 0, stream>>>(a, pairs, ntx, per_cta, lanes_16);
     return cudaGetLastError();
 }
 
@@ -174,21 +181,20 @@ cudaError_t launch_linear_volume(const ProjArgs& a, cudaStream_t stream) {
 // sample's cell and the next one's share a z plane: its sum over y and x (the inner part of the sample's
 // sum, in its order) is kept, and each sample but the first reads two pair rows instead of four.
 // 1000 slices of 256^2 with 7 offsets and weights: 1417 us -> 1192 us (1113 us with the offsets tabulated
-// beside their window values).
+// beside their window values, 1067 us with the padded copy).
 template<bool OUT_C>
 __global__ void __launch_bounds__(EXTRACT_THREADS)
 extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx) {
     const int wp = a.slice_w / 2 + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y0 = (blockIdx.x / ntx) * (TY * PAIR_PPT) + (warp >> 1) * 4 + (lane >> 3);
-    const int u = (blockIdx.x % ntx) * TX + (warp & 1) * 8 + (lane & 7);
+    const int y0 = (blockIdx.x / ntx) * (TY * PAIR_PPT) + (warp >> 1) * 4 + pair_row(lane);
+    const int u = (blockIdx.x % ntx) * TX + (warp & 1) * 8 + pair_column(lane);
     __shared__ float2 s_w[W_TABLE];
     fill_w_table(a, s_w);
     if (u >= wp)
         return;
     const Spectrum3 sp{a.vol_d, a.vol_h, a.vol_w, a.in_centered};
-    const int WP = a.vol_w / 2 + 1;
-    const int sz = a.vol_h * WP, sy = WP;
+    const int sz = a.pair_sz, sy = a.pair_sy;
     const int lo0 = -sp.n0 / 2, hi0 = (sp.n0 - 1) / 2;
     const bool has_out_w = a.out_w.present;
     const float f1 = div(static_cast<float>(u), a.f_slice1);
@@ -251,14 +257,14 @@ bool use_pairs(const ProjArgs& a) {
     const int64_t pix = a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
     ProjArgs plain = a;
     plain.wsize = 1;  // the w-windowed form reads the pair copy too (extract_pairs_w_kernel)
-    return pairs_apply(plain) && pix >= 2 * vox;
+    return pairs_apply(plain) && pairs_pay(pix * (a.wsize > 1 ? a.wsize : 1), vox);
 }
 
-cudaError_t launch_pairs(const ProjArgs& a, cudaStream_t stream, bool& done) {
+cudaError_t launch_pairs(const ProjArgs& call, cudaStream_t stream, bool& done) {
     done = false;
-    const int64_t wp_vol = a.vol_w / 2 + 1;
-    const int64_t vox = static_cast<int64_t>(a.vol_d) * a.vol_h * wp_vol;
-    float4* pairs = static_cast<float4*>(scratch_alloc(static_cast<size_t>(vox) * sizeof(float4), stream));
+    ProjArgs a = call;
+    pad_pairs(a);
+    float4* pairs = static_cast<float4*>(scratch_alloc(static_cast<size_t>(pair_elements(a)) * sizeof(float4), stream));
     if (!pairs)
         return cudaSuccess; // no scratch: the caller takes the generic path
     launch_make_pairs(a, pairs, stream);
@@ -415,6 +421,8 @@ cudaError_t launch_make_pairs(const ProjArgs& a, float4* pairs, cudaStream_t str
         return cudaLaunchKernelEx(&cfg, make_pairs<uint32_t>, a, pairs);
     return cudaLaunchKernelEx(&cfg, make_pairs<int64_t>, a, pairs);
 }
+
+cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream) { return launch_interp<I_LINEAR>(a, stream); }
 
 cudaError_t launch_extract(const ProjArgs& a, cudaStream_t stream) {
     if (a.n_slices > 0 && use_pairs(a)) {

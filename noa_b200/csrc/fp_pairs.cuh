@@ -1,6 +1,6 @@
 // Pair copy of a volume for LINEAR extraction, shared by the per-call and batched extraction kernels.
 //
-// The copy is dense (D x H x W/2+1) and element (z, y, x) holds the two x-neighbours v[z][y][x] and
+// Element (z, y, x) of the copy (D x H x W/2+1, strides pair_sz, pair_sy, 1) holds the two x-neighbours v[z][y][x] and
 // v[z][y][x+1] (zero past the last column) as one float4, so the 2x2x2 trilinear cell is 4 aligned
 // 16-byte loads instead of 8 scattered 8-byte ones. The taps, weights and summation order are those of
 // interp_linear_3d, so results are bit-identical to the generic path.
@@ -112,23 +112,71 @@ struct PairPlane {
     }
 };
 
+// Strides of a pair copy. Dense for the copies that callers hold (nb_volume_pairs). Copies that the library
+// makes for itself pad rows to 4 and planes to 2 elements past a multiple of 8: the L1 serves eight 16-byte
+// lanes at a time, each element in one of eight bank groups, and with these strides the 2 x 4 pixels that
+// share a pass fall on 1.96 lines of a group on average over orientations, against 2.69 for 1 x 8 pixels
+// over dense planes of an even number of rows, all of which start on the same banks (replayed on the CPU; the
+// best of the 64 pairs of strides modulo 8). The L1's wavefronts are what bounds the extraction: 4096 slices
+// of 256^3 1165 us -> 1104 us, with the matrix read once per slice and column (LeanColumn).
+inline void dense_pairs(ProjArgs& a) {
+    a.pair_sy = a.vol_w / 2 + 1;
+    a.pair_sz = static_cast<int>(static_cast<int64_t>(a.vol_h) * a.pair_sy);  // pairs_apply bounds it
+}
+
+inline void pad_pairs(ProjArgs& a) {
+    const int64_t sy = (a.vol_w / 2 + 1 + 3) / 8 * 8 + 4;
+    const int64_t sz = (a.vol_h * sy + 5) / 8 * 8 + 2;
+    if (sz * a.vol_d < (int64_t(1) << 31)) {
+        a.pair_sy = static_cast<int>(sy);
+        a.pair_sz = static_cast<int>(sz);
+    }
+}
+
+inline int64_t pair_elements(const ProjArgs& a) { return static_cast<int64_t>(a.vol_d) * a.pair_sz; }
+
+// Row and column of a lane within its warp's 4 x 8 pixels: 2 x 4 per eight lanes.
+__device__ __forceinline__ int pair_row(int lane) { return (lane >> 4) * 2 + ((lane >> 2) & 1); }
+__device__ __forceinline__ int pair_column(int lane) { return ((lane >> 3) & 1) * 4 + (lane & 3); }
+
 // slice2grid for a Mat33 rotation with no scaling and no Ewald curvature, when the slice's matrix
 // column 0 is finite: rotate() computes ((m_k0 * 0) + (m_k1 * f0)) + (m_k2 * f1), and for finite m_k0
 // the first product is a zero whose sign never reaches the result (the coordinates then decide the
-// cutoff, the cell, its weights and the Friedel flip the same way), so it is left out.
-__device__ __forceinline__ void slice2grid_lean(const float* m, float f0, float f1, float& z, float& y, float& x) {
-    z = add(mul(m[1], f0), mul(m[2], f1));
-    y = add(mul(m[4], f0), mul(m[5], f1));
-    x = add(mul(m[7], f0), mul(m[8], f1));
-}
+// cutoff, the cell, its weights and the Friedel flip the same way), so it is left out. The products with
+// f1 are those of a column of pixels.
+struct LeanColumn {
+    float z1, y1, x1, z2, y2, x2;
 
-// Whether slice b of `a` can take slice2grid_lean; `m` is then its matrix.
-__device__ __forceinline__ bool lean_rotation(const ProjArgs& a, int64_t b, const float*& m) {
-    if (a.rot.kind != 2 || a.scale.kind != 0 || a.ews.on)
-        return false;
-    m = xform_ptr(a.rot, b, 12);
-    return isfinite(m[0]) && isfinite(m[3]) && isfinite(m[6]);
-}
+    // Whether slice b of `a` can take the lean form. The matrix is read once, 16 bytes at a time (its 48
+    // bytes are aligned): read per pixel it cost as many L1 wavefronts as one of the four tap loads.
+    __device__ __forceinline__ bool load(const ProjArgs& a, int64_t b, float f1) {
+        if (a.rot.kind != 2 || a.scale.kind != 0 || a.ews.on)
+            return false;
+        const float* m = xform_ptr(a.rot, b, 12);
+        float m0, m2, m3, m5, m6, m8;
+        if (a.rot.data) {
+            const float4* rows = reinterpret_cast<const float4*>(m);
+            const float4 r0 = __ldg(rows), r1 = __ldg(rows + 1);
+            m0 = r0.x; z1 = r0.y; m2 = r0.z; m3 = r0.w;
+            y1 = r1.x; m5 = r1.y; m6 = r1.z; x1 = r1.w;
+            m8 = __ldg(m + 8);
+        } else {
+            m0 = m[0]; z1 = m[1]; m2 = m[2]; m3 = m[3];
+            y1 = m[4]; m5 = m[5]; m6 = m[6]; x1 = m[7];
+            m8 = m[8];
+        }
+        z2 = mul(m2, f1);
+        y2 = mul(m5, f1);
+        x2 = mul(m8, f1);
+        return isfinite(m0) && isfinite(m3) && isfinite(m6);
+    }
+
+    __device__ __forceinline__ void at(float f0, float& z, float& y, float& x) const {
+        z = add(mul(z1, f0), z2);
+        y = add(mul(y1, f0), y2);
+        x = add(mul(x1, f0), x2);
+    }
+};
 
 // Whether a call may read the pair copy: LINEAR, complex volume given as an array, no input weights,
 // no w-window (per-call extractions take extract_pairs_w_kernel for that), a copy addressable in 32
@@ -139,6 +187,18 @@ inline bool pairs_apply(const ProjArgs& a) {
     return a.interp == I_LINEAR && a.in_cplx && !a.in_w.present && !a.in.is_value && a.wsize <= 1 &&
            vox < (int64_t(1) << 31);
 }
+
+// From how many output pixels on a LINEAR extraction is faster through a pair copy made for it: three per
+// voxel, four where the copy is twice the L2 and more (2^24 voxels), and 2 M. Measured without and with, us:
+// 64^3 x 256 slices (4 pixels per voxel) 15 and 17; 128^3 x 256 (2) 34 and 35, x 384 (3) 45 and 41; 200^3 x 400 (2)
+// 93 and 101, x 600 (3) 135 and 129; 256^3 x 512 (2) 196 and 196, x 768 (3) 276 and 243; 384^3 x 1152 (3) 959 and
+// 962, x 1536 (4) 1328 and 1253; 512^3 x 1536 (3) 2489 and 2622, x 2048 (4) 3349 and 3390, x 4096 (8) 6778 and 6473.
+inline bool pairs_pay(int64_t pixels, int64_t voxels) {
+    return pixels >= (voxels < (int64_t(1) << 24) ? 3 : 4) * voxels && pixels >= (int64_t(1) << 21);
+}
+
+// The per-call LINEAR extraction from the volume itself (no w-window).
+cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream);
 
 // Writes the pair copy of a.in (a.vol_d x a.vol_h x a.vol_w/2+1 complex values) to `pairs`. With
 // `priority`, the launch carries that scheduling priority (kept by a graph captured from it).

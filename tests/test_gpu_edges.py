@@ -82,3 +82,29 @@ def test_pair_queue(kw):
                          ids=["pairs", "beyond", "weights", "power", "real"])
 def test_linear_extraction_groups(kw, remap):
     _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5)
+
+
+# The rule on making a pair copy (three pixels per voxel, 2 M pixels), its padded strides, and requests of a
+# batch that read their volume in grids of their own: the same bits with and without the copy.
+@pytest.mark.parametrize("n,size,count", [(33, 33, 4000), (64, 64, 1100), (96, 95, 470), (40, 200, 110), (128, 128, 250)])
+def test_extraction_with_and_without_pair_copy(n, size, count):
+    import torch
+    from noa_b200 import fourier_project as fp, synthetic
+    from noa_b200.batch import ExtractBatch, ExtractRequest
+    vol = torch.from_numpy(synthetic.make_volume(n, seed=n)).cuda()
+    rot = fp.pack_rotations(torch.from_numpy(synthetic.random_rotations(count, seed=count)).cuda())
+    shape, slices = (1, n, n, n), (count, 1, size, size)
+    outs = [torch.empty((count, 1, size, size // 2 + 1), dtype=torch.complex64, device="cuda") for _ in range(3)]
+    try:
+        for out, limit in zip(outs, (None, 0)):
+            fp.set_scratch_limit(limit)
+            fp.extract_central_slices_3d("hc2h", vol, None, shape, out, None, slices, None, rot)
+    finally:
+        fp.set_scratch_limit(None)
+    batch = ExtractBatch("hc2h", [ExtractRequest(volume=vol, volume_shape=shape, slice=outs[2], slice_shape=slices,
+                                                 fwd_rotation=rot)], autotune=False)
+    batch.run()
+    torch.cuda.synchronize()
+    assert batch.info()["n_direct"] == 1
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    batch.close()

@@ -105,8 +105,6 @@ __device__ __forceinline__ int frequency2index(bool centered, int f, int n) {
 // ---------------------------------------------------------------------------------------------------
 // Transforms (Transform.hpp:201-218, Mat.hpp:420-424, Quaternion.hpp:167-181).
 // ---------------------------------------------------------------------------------------------------
-struct Mat33 { float m[9]; };
-struct Quat { float z, y, x, w; };
 
 __device__ __forceinline__ const float* xform_ptr(const XformView& x, int64_t batch, int stride) {
     if (!x.data)
@@ -385,75 +383,6 @@ struct SliceReader {
     }
 };
 
-// ---------------------------------------------------------------------------------------------------
-// interpolate_spectrum, 3-D (volume) form. `freq` is in samples, centered on DC.
-// ---------------------------------------------------------------------------------------------------
-template<int I, bool CPLX>
-__device__ __forceinline__ float2 interp_spectrum_3d(const SrcView& src, const Spectrum3& sp,
-                                                     float f0, float f1, float f2) {
-    constexpr int SIZE = InterpTraits<I>::SIZE;
-    constexpr bool FLIP_EARLY = SIZE <= 2;
-    const int lo0 = -sp.n0 / 2, hi0 = (sp.n0 - 1) / 2;
-    const int lo1 = -sp.n1 / 2, hi1 = (sp.n1 - 1) / 2;
-    const int hi2 = sp.n2 / 2;
-    float conjugate = 1.f;
-    if (FLIP_EARLY && f2 < 0.f) {
-        f0 = -f0; f1 = -f1; f2 = -f2;
-        conjugate = -1.f;
-    }
-    if constexpr (I == I_NEAREST) {
-        // NEAREST returns before the early-flip conjugation (Interpolation.hpp:480-485).
-        const int i0 = static_cast<int>(roundf(f0));
-        const int i1 = static_cast<int>(roundf(f1));
-        const int i2 = static_cast<int>(roundf(f2));
-        float2 v = make_float2(0.f, 0.f);
-        if (i0 >= lo0 && i0 <= hi0 && i1 >= lo1 && i1 <= hi1 && i2 >= 0 && i2 <= hi2)
-            v = src_read<CPLX>(src, frequency2index(sp.centered, i0, sp.n0),
-                               frequency2index(sp.centered, i1, sp.n1), i2);
-        return v;
-    } else {
-        constexpr int START = -(SIZE - 1) / 2;
-        const float fl0 = floorf(f0), fl1 = floorf(f1), fl2 = floorf(f2);
-        const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1), b2 = static_cast<int>(fl2);
-        float w0[SIZE], w1[SIZE], w2[SIZE];
-        interp_weights<I>(sub(f0, fl0), w0);
-        interp_weights<I>(sub(f1, fl1), w1);
-        interp_weights<I>(sub(f2, fl2), w2);
-        float2 value = make_float2(0.f, 0.f);
-        // Windows of 6 and 8 taps keep the z loop rolled: 216/512 unrolled taps only cost registers
-        // and compile time, these modes are arithmetic-bound either way.
-#pragma unroll (SIZE <= 4 ? SIZE : 1)
-        for (int z = 0; z < SIZE; ++z) {
-            float2 vz = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int y = 0; y < SIZE; ++y) {
-                float2 vy = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int x = 0; x < SIZE; ++x) {
-                    int t0 = b0 + START + z, t1 = b1 + START + y, t2 = b2 + START + x;
-                    float conj = 1.f;
-                    if (!FLIP_EARLY && t2 < 0) {
-                        t0 = -t0; t1 = -t1; t2 = -t2;
-                        conj = -1.f;
-                    }
-                    if (t0 >= lo0 && t0 <= hi0 && t1 >= lo1 && t1 <= hi1 && t2 >= 0 && t2 <= hi2) {
-                        float2 v = src_read<CPLX>(src, frequency2index(sp.centered, t0, sp.n0),
-                                                  frequency2index(sp.centered, t1, sp.n1), t2);
-                        if (!FLIP_EARLY)
-                            v.y *= conj;
-                        vy = cfma(v, w2[x], vy);
-                    }
-                }
-                vz = cfma(vy, w1[y], vz);
-            }
-            value = cfma(vz, w0[z], value);
-        }
-        if (FLIP_EARLY)
-            value.y *= conjugate;
-        return value;
-    }
-}
-
 // interpolate_spectrum, 2-D (slice) form; `batch` selects the slice.
 template<int I, bool CPLX>
 __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const Spectrum2& sp, int64_t batch,
@@ -642,127 +571,26 @@ __device__ __forceinline__ float2 interp_linear_3d(const View3<Idx>& v, const Sp
     return value;
 }
 
-// Generic interpolate_spectrum, 3-D, on a View3 (any window).
+// interpolate_spectrum, 3-D, on a View3: NEAREST and LINEAR (the wider windows: fp_window.cuh).
 template<int I, bool CPLX, typename Idx>
 __device__ __forceinline__ float2 interp_3d(const View3<Idx>& v, const Spectrum3& sp, float f0, float f1, float f2) {
+    static_assert(I == I_NEAREST || I == I_LINEAR, "the wider windows are interpolated by lane groups");
     if constexpr (I == I_LINEAR) {
         return interp_linear_3d<CPLX>(v, sp, f0, f1, f2);
     } else {
-        constexpr int SIZE = InterpTraits<I>::SIZE;
-        constexpr bool FLIP_EARLY = SIZE <= 2;
-        const int lo0 = -sp.n0 / 2, hi0 = (sp.n0 - 1) / 2;
-        const int lo1 = -sp.n1 / 2, hi1 = (sp.n1 - 1) / 2;
-        const int hi2 = sp.n2 / 2;
-        float conjugate = 1.f;
-        if (FLIP_EARLY && f2 < 0.f) {
+        // NEAREST returns before the early-flip conjugation (Interpolation.hpp:480-485).
+        if (f2 < 0.f) {
             f0 = -f0; f1 = -f1; f2 = -f2;
-            conjugate = -1.f;
         }
-        if constexpr (I == I_NEAREST) {
-            // NEAREST returns before the early-flip conjugation (Interpolation.hpp:480-485).
-            const int i0 = static_cast<int>(roundf(f0));
-            const int i1 = static_cast<int>(roundf(f1));
-            const int i2 = static_cast<int>(roundf(f2));
-            float2 r = make_float2(0.f, 0.f);
-            if (i0 >= lo0 && i0 <= hi0 && i1 >= lo1 && i1 <= hi1 && i2 >= 0 && i2 <= hi2)
-                r = view_read<CPLX>(v, static_cast<Idx>(frequency2index(sp.centered, i0, sp.n0)) * v.s0 +
-                                       static_cast<Idx>(frequency2index(sp.centered, i1, sp.n1)) * v.s1 +
-                                       static_cast<Idx>(i2) * v.s2);
-            return r;
-        } else {
-            constexpr int START = -(SIZE - 1) / 2;
-            const float fl0 = floorf(f0), fl1 = floorf(f1), fl2 = floorf(f2);
-            const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1), b2 = static_cast<int>(fl2);
-            float w0[SIZE], w1[SIZE], w2[SIZE];
-            interp_weights<I>(sub(f0, fl0), w0);
-            interp_weights<I>(sub(f1, fl1), w1);
-            interp_weights<I>(sub(f2, fl2), w2);
-            float2 value = make_float2(0.f, 0.f);
-            constexpr int END = SIZE / 2;
-            // Interior fast path: every tap in bounds and on the stored half (no per-tap Friedel
-            // flip), so each (z, y) row of the window is SIZE consecutive x elements. Same terms in the
-            // same order as the general loop below, hence the same bits.
-            if (b0 + START >= lo0 && b0 + END <= hi0 && b1 + START >= lo1 && b1 + END <= hi1 &&
-                b2 + START >= 0 && b2 + END <= hi2) {
-                const Idx x0 = static_cast<Idx>(b2 + START) * v.s2;
-                // With contiguous x and a 16-byte aligned volume, a row of SIZE complex values is read
-                // as SIZE/2 aligned 16-byte loads from the even element at or before its start, plus
-                // one 8-byte load when the start is odd: fewer, wider loads than SIZE 8-byte ones.
-                constexpr bool WIDE = CPLX && SIZE % 2 == 0;
-                const bool wide = WIDE && v.s2 == 1 && (reinterpret_cast<uintptr_t>(v.data) & 15) == 0;
-#pragma unroll (SIZE <= 4 ? SIZE : 1)
-                for (int z = 0; z < SIZE; ++z) {
-                    const Idx oz = static_cast<Idx>(frequency2index(sp.centered, b0 + START + z, sp.n0)) * v.s0 + x0;
-                    float2 vz = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int y = 0; y < SIZE; ++y) {
-                        const Idx row = oz + static_cast<Idx>(frequency2index(sp.centered, b1 + START + y, sp.n1)) * v.s1;
-                        float2 vy = make_float2(0.f, 0.f);
-                        if constexpr (WIDE) {
-                            if (wide) {
-                                const bool odd = (row & 1) != 0;
-                                const float2* e = static_cast<const float2*>(v.data) + (row - (odd ? 1 : 0));
-                                float4 q[SIZE / 2];
-#pragma unroll
-                                for (int j = 0; j < SIZE / 2; ++j)
-                                    q[j] = ldg_evict_last_half(reinterpret_cast<const float4*>(e) + j);
-                                const float2 last = odd ? __ldg(e + SIZE) : make_float2(0.f, 0.f);
-#pragma unroll
-                                for (int x = 0; x < SIZE; ++x) {
-                                    // element x of the row: element x + odd of the loaded run
-                                    const int i0 = x, i1 = x + 1;
-                                    const float2 even = (i0 & 1) ? make_float2(q[i0 / 2].z, q[i0 / 2].w)
-                                                                 : make_float2(q[i0 / 2].x, q[i0 / 2].y);
-                                    const float2 shifted = i1 == SIZE ? last
-                                        : ((i1 & 1) ? make_float2(q[i1 / 2].z, q[i1 / 2].w)
-                                                    : make_float2(q[i1 / 2].x, q[i1 / 2].y));
-                                    vy = cfma(odd ? shifted : even, w2[x], vy);
-                                }
-                                vz = cfma(vy, w1[y], vz);
-                                continue;
-                            }
-                        }
-#pragma unroll
-                        for (int x = 0; x < SIZE; ++x)
-                            vy = cfma(view_read<CPLX>(v, row + static_cast<Idx>(x) * v.s2), w2[x], vy);
-                        vz = cfma(vy, w1[y], vz);
-                    }
-                    value = cfma(vz, w0[z], value);
-                }
-                return value;
-            }
-#pragma unroll 1
-            for (int z = 0; z < SIZE; ++z) {
-                float2 vz = make_float2(0.f, 0.f);
-#pragma unroll (SIZE <= 4 ? SIZE : 1)
-                for (int y = 0; y < SIZE; ++y) {
-                    float2 vy = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int x = 0; x < SIZE; ++x) {
-                        int t0 = b0 + START + z, t1 = b1 + START + y, t2 = b2 + START + x;
-                        float conj = 1.f;
-                        if (!FLIP_EARLY && t2 < 0) {
-                            t0 = -t0; t1 = -t1; t2 = -t2;
-                            conj = -1.f;
-                        }
-                        if (t0 >= lo0 && t0 <= hi0 && t1 >= lo1 && t1 <= hi1 && t2 >= 0 && t2 <= hi2) {
-                            float2 val = view_read<CPLX>(
-                                v, static_cast<Idx>(frequency2index(sp.centered, t0, sp.n0)) * v.s0 +
-                                   static_cast<Idx>(frequency2index(sp.centered, t1, sp.n1)) * v.s1 +
-                                   static_cast<Idx>(t2) * v.s2);
-                            if (!FLIP_EARLY)
-                                val.y *= conj;
-                            vy = cfma(val, w2[x], vy);
-                        }
-                    }
-                    vz = cfma(vy, w1[y], vz);
-                }
-                value = cfma(vz, w0[z], value);
-            }
-            if (FLIP_EARLY)
-                value.y *= conjugate;
-            return value;
-        }
+        const int i0 = static_cast<int>(roundf(f0));
+        const int i1 = static_cast<int>(roundf(f1));
+        const int i2 = static_cast<int>(roundf(f2));
+        float2 r = make_float2(0.f, 0.f);
+        if (i0 >= -sp.n0 / 2 && i0 <= (sp.n0 - 1) / 2 && i1 >= -sp.n1 / 2 && i1 <= (sp.n1 - 1) / 2 && i2 >= 0 && i2 <= sp.n2 / 2)
+            r = view_read<CPLX>(v, static_cast<Idx>(frequency2index(sp.centered, i0, sp.n0)) * v.s0 +
+                                   static_cast<Idx>(frequency2index(sp.centered, i1, sp.n1)) * v.s1 +
+                                   static_cast<Idx>(i2) * v.s2);
+        return r;
     }
 }
 

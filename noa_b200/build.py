@@ -4,18 +4,20 @@
 
 Each .cu under noa_b200/csrc is compiled with nvcc for sm_100a (-gencode arch=compute_100a,code=sm_100a)
 in parallel, then linked into one shared library with the CUDA runtime linked statically, so it loads
-beside any PyTorch build; noa_b200/_lib/_marshal.so is the Python API's native marshalling. Rebuilds only
-what changed.
+beside any PyTorch build; noa_b200/_lib/_marshal.<ABI tag>.so is the Python API's native marshalling, for the
+Python that builds it. Rebuilds only what changed.
 """
 from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import importlib.machinery
 import os
 import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -24,6 +26,7 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libnoa_b200.so")
+MARSHAL = "_marshal" + importlib.machinery.EXTENSION_SUFFIXES[0]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
@@ -67,9 +70,10 @@ def _compile(src: str, verbose_ptxas: bool) -> tuple[str, str]:
 
 
 def _build_marshal() -> None:
-    """The Python API's native marshalling (csrc/marshal.c). Without Python's headers the API marshals
-    through ctypes instead."""
-    src, out = os.path.join(CSRC, "marshal.c"), os.path.join(LIBDIR, "_marshal.so")
+    """The Python API's native marshalling (csrc/marshal.c). It uses the whole CPython API, so its name carries
+    the ABI tag of the Python it is built for and no other loads it. Without it (no Python headers, or it does
+    not compile) the API marshals through ctypes instead."""
+    src, out = os.path.join(CSRC, "marshal.c"), os.path.join(LIBDIR, MARSHAL)
     include = sysconfig.get_paths()["include"]
     if not os.path.exists(os.path.join(include, "Python.h")) or not _stale(out, [src] + _headers()):
         return
@@ -77,7 +81,8 @@ def _build_marshal() -> None:
            src, "-o", out]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"building {src} failed:\n{r.stdout}\n{r.stderr}")
+        warnings.warn(f"building {src} failed, calls will be marshalled through ctypes:\n{r.stdout}\n{r.stderr}",
+                      RuntimeWarning)
 
 
 def build(verbose_ptxas: bool = False, jobs: int | None = None) -> str:

@@ -14,6 +14,7 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import warnings
 from dataclasses import dataclass
 
 import numpy as np
@@ -276,25 +277,31 @@ def _ref(x):
 
 
 # ---------------------------------------------------------------------------------------------------
-# Calls: natively (csrc/marshal.c, built beside the library), or through the ctypes structures where that
-# module was not built (no Python headers). Both fill the same structures from the same arguments.
+# Calls: natively (csrc/marshal.c, built beside the library), or through the ctypes structures where there is
+# no such module for this interpreter (built without Python headers, or under another Python: its file name
+# carries the interpreter's ABI tag) or where it does not load. Both fill the same structures from the same
+# arguments.
 # ---------------------------------------------------------------------------------------------------
-_MARSHAL_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_marshal.so")
+_MARSHAL_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_marshal" + importlib.machinery.EXTENSION_SUFFIXES[0])
 _native_module: list = []
 _ADDRESSES: dict = {}
 
 
 def _native():
-    """The marshalling module, or None if it was not built."""
+    """The marshalling module, or None if there is none for this interpreter or it does not load."""
     if not _native_module:
         module = None
         if os.path.exists(_MARSHAL_PATH):
-            loader = importlib.machinery.ExtensionFileLoader("_marshal", _MARSHAL_PATH)
-            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_marshal", loader))
-            loader.exec_module(module)
             torch = _torch()
             _fill_dtypes()
-            module.init(NoaB200Error, _DTYPES, INTERPS, as_nb_transform, torch.float32, torch.Tensor)
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("_marshal", _MARSHAL_PATH)
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_marshal", loader))
+                loader.exec_module(module)
+                module.init(NoaB200Error, _DTYPES, INTERPS, as_nb_transform, torch.float32, torch.Tensor)
+            except ImportError as e:
+                module = None
+                warnings.warn(f"calls are marshalled through ctypes: {e}", RuntimeWarning)
         _native_module.append(module)
     return _native_module[0]
 

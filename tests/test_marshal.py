@@ -1,10 +1,14 @@
 """The native marshalling fills the structures that the ctypes path fills, and refuses what it refuses (CPU)."""
 import ctypes as C
+import os
+import subprocess
+import sysconfig
 
 import numpy as np
 import pytest
 import torch
 
+from noa_b200 import build
 from noa_b200 import fourier_project as fp
 
 pytestmark = pytest.mark.skipif(fp._native() is None, reason="built without Python headers")
@@ -89,3 +93,26 @@ def test_same_refusals(monkeypatch, change):
             _seen(monkeypatch, native, call, 2)
         errors.append((type(e.value), getattr(e.value, "code", None)))
     assert errors[0] == errors[1]
+
+
+def test_the_module_is_of_this_interpreter():
+    """Its name carries the ABI tag, so a module that another Python built beside the library is not loaded."""
+    assert fp._MARSHAL_PATH.endswith("/_marshal" + sysconfig.get_config_var("EXT_SUFFIX"))
+    assert build.MARSHAL == os.path.basename(fp._MARSHAL_PATH)
+
+
+def test_a_module_that_does_not_load_leaves_ctypes(monkeypatch, tmp_path):
+    path = tmp_path / build.MARSHAL
+    path.write_bytes(b"not an extension")
+    monkeypatch.setattr(fp, "_MARSHAL_PATH", str(path))
+    monkeypatch.setattr(fp, "_native_module", [])
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        assert fp._native() is None
+    assert fp._native() is None  # decided once, without another warning
+
+
+def test_a_module_that_does_not_compile_leaves_the_library_build_going(monkeypatch, tmp_path):
+    monkeypatch.setattr(build, "LIBDIR", str(tmp_path))
+    monkeypatch.setattr(build.subprocess, "run", lambda *a, **k: subprocess.CompletedProcess(a, 1, "", "no compiler"))
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        build._build_marshal()

@@ -13,7 +13,7 @@
 
 #include "noa_b200/fourier_project.h"
 
-static PyObject *g_error, *g_dtypes, *g_interps, *g_transform_helper, *g_float32, *g_tensor; /* from init() */
+static PyObject *g_error, *g_dtypes, *g_interps, *g_transform_helper, *g_ews_helper, *g_float32, *g_tensor; /* from init() */
 static PyObject *s_data_ptr, *s_dtype, *s_shape, *s_stride, *s_is_contiguous, *s_fftfreq_sinc, *s_fftfreq_blackman;
 
 static int fail(long code, const char* message) {
@@ -197,6 +197,30 @@ static int to_window(PyObject* w, double* sinc, double* blackman) {
     return st;
 }
 
+/* One number, or a pair of them as a tuple; anything else (an array, a tensor) through the helper. */
+static int to_ews_radius(PyObject* ews, double out[2]) {
+    if (PyFloat_CheckExact(ews) || PyLong_CheckExact(ews)) {
+        const int st = to_double(ews, &out[0]);
+        out[1] = out[0];
+        return st;
+    }
+    PyObject* pair;
+    if (PyTuple_CheckExact(ews)) {
+        pair = Py_NewRef(ews);
+    } else {
+        pair = PyObject_CallOneArg(g_ews_helper, ews);
+        if (!pair)
+            return -1;
+    }
+    int st = PyTuple_Check(pair) && PyTuple_GET_SIZE(pair) >= 2 ? 0 : -1;
+    if (st != 0)
+        PyErr_SetString(PyExc_IndexError, "ews_radius: two numbers are expected");
+    for (int i = 0; st == 0 && i < 2; ++i)
+        st = to_double(PyTuple_GET_ITEM(pair, i), &out[i]);
+    Py_DECREF(pair);
+    return st;
+}
+
 /* (interp, fftfreq_cutoff, target_shape, ews_radius, windowed_sinc, w_windowed_sinc, add_to_output,
  * correct_weights) */
 static int to_options(PyObject* o, nb_options* out) {
@@ -226,26 +250,8 @@ static int to_options(PyObject* o, nb_options* out) {
     PyObject* target = PyTuple_GET_ITEM(o, 2);
     if (target != Py_None && to_int64s(target, out->target_shape, 4, HEAD) != 0)
         return -1;
-    PyObject* ews = PyTuple_GET_ITEM(o, 3);
-    if (PyTuple_CheckExact(ews) && PyTuple_GET_SIZE(ews) >= 2) {
-        if (to_double(PyTuple_GET_ITEM(ews, 0), &out->ews_radius[0]) != 0 ||
-            to_double(PyTuple_GET_ITEM(ews, 1), &out->ews_radius[1]) != 0)
-            return -1;
-    } else if (PySequence_Check(ews)) {
-        for (int i = 0; i < 2; ++i) {
-            PyObject* v = PySequence_GetItem(ews, i);
-            if (!v)
-                return -1;
-            const int st = to_double(v, &out->ews_radius[i]);
-            Py_DECREF(v);
-            if (st != 0)
-                return -1;
-        }
-    } else {
-        if (to_double(ews, &out->ews_radius[0]) != 0)
-            return -1;
-        out->ews_radius[1] = out->ews_radius[0];
-    }
+    if (to_ews_radius(PyTuple_GET_ITEM(o, 3), out->ews_radius) != 0)
+        return -1;
     if (to_window(PyTuple_GET_ITEM(o, 4), &out->fftfreq_sinc, &out->fftfreq_blackman) != 0 ||
         to_window(PyTuple_GET_ITEM(o, 5), &out->w_fftfreq_sinc, &out->w_fftfreq_blackman) != 0)
         return -1;
@@ -316,15 +322,17 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     return PyLong_FromLong(code);
 }
 
-/* init(error class, {dtype: code}, {interp: code}, transform helper, torch.float32, torch.Tensor) */
+/* init(error class, {dtype: code}, {interp: code}, transform helper, ews_radius helper, torch.float32,
+ *      torch.Tensor) */
 static PyObject* init(PyObject* self, PyObject* args) {
     (void) self;
-    PyObject *error, *dtypes, *interps, *helper, *float32, *tensor;
-    if (!PyArg_ParseTuple(args, "OO!O!OOO", &error, &PyDict_Type, &dtypes, &PyDict_Type, &interps, &helper, &float32, &tensor))
+    PyObject *error, *dtypes, *interps, *helper, *ews, *float32, *tensor;
+    if (!PyArg_ParseTuple(args, "OO!O!OOOO", &error, &PyDict_Type, &dtypes, &PyDict_Type, &interps, &helper, &ews,
+                          &float32, &tensor))
         return NULL;
-    PyObject** to[6] = {&g_error, &g_dtypes, &g_interps, &g_transform_helper, &g_float32, &g_tensor};
-    PyObject* from[6] = {error, dtypes, interps, helper, float32, tensor};
-    for (int i = 0; i < 6; ++i) {
+    PyObject** to[7] = {&g_error, &g_dtypes, &g_interps, &g_transform_helper, &g_ews_helper, &g_float32, &g_tensor};
+    PyObject* from[7] = {error, dtypes, interps, helper, ews, float32, tensor};
+    for (int i = 0; i < 7; ++i) {
         Py_INCREF(from[i]);
         Py_XSETREF(*to[i], from[i]);
     }

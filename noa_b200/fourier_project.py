@@ -228,6 +228,13 @@ def _default_options() -> NbOptions:
     return _DEFAULT_OPTIONS[0]
 
 
+def _ews_pair(ews_radius) -> tuple[float, float]:
+    """The two radii of a number (both) or of anything with two elements."""
+    if isinstance(ews_radius, (int, float)) or np.isscalar(ews_radius):
+        ews_radius = (ews_radius, ews_radius)
+    return float(ews_radius[0]), float(ews_radius[1])
+
+
 def _options(interp="linear", fftfreq_cutoff=0.5, target_shape=None, ews_radius=(0.0, 0.0),
              windowed_sinc: WindowedSinc | None = None, w_windowed_sinc: WindowedSinc | None = None,
              add_to_output=False, correct_weights=False) -> NbOptions:
@@ -237,9 +244,7 @@ def _options(interp="linear", fftfreq_cutoff=0.5, target_shape=None, ews_radius=
     if target_shape is not None:
         for i in range(4):
             o.target_shape[i] = int(target_shape[i])
-    if isinstance(ews_radius, (int, float)) or np.isscalar(ews_radius):
-        ews_radius = (ews_radius, ews_radius)
-    o.ews_radius[0], o.ews_radius[1] = float(ews_radius[0]), float(ews_radius[1])
+    o.ews_radius[0], o.ews_radius[1] = _ews_pair(ews_radius)
     ws = windowed_sinc or _NO_WINDOW
     wws = w_windowed_sinc or _NO_WINDOW
     o.fftfreq_sinc, o.fftfreq_blackman = float(ws.fftfreq_sinc), float(ws.fftfreq_blackman)
@@ -298,7 +303,7 @@ def _native():
                 loader = importlib.machinery.ExtensionFileLoader("_marshal", _MARSHAL_PATH)
                 module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_marshal", loader))
                 loader.exec_module(module)
-                module.init(NoaB200Error, _DTYPES, INTERPS, as_nb_transform, torch.float32, torch.Tensor)
+                module.init(NoaB200Error, _DTYPES, INTERPS, as_nb_transform, _ews_pair, torch.float32, torch.Tensor)
             except ImportError as e:
                 module = None
                 warnings.warn(f"calls are marshalled through ctypes: {e}", RuntimeWarning)

@@ -66,6 +66,30 @@ def test_same_structures(monkeypatch, volume, weight, rotation, kw):
         assert a == b and len(a) == 1
 
 
+def _call_with(**kw):
+    fp.extract_central_slices_3d("hc2h", _vol, None, (1, 8, 8, 8), _out, None, (3, 1, 8, 8), None, _packed, stream=3, **kw)
+
+
+def _same(monkeypatch, call):
+    """What both ways make of `call`: the structures, or the class of the error."""
+    results = []
+    for native in (True, False):
+        try:
+            results.append(_seen(monkeypatch, native, call, 2))
+        except Exception as e:
+            results.append(type(e))
+    return results
+
+
+@pytest.mark.parametrize("radius,accepted", [
+    (0, True), (3.5, True), (True, True), (np.float32(3), True), (np.int64(4), True), ((1, 2), True), ([1.5, 2], True),
+    ((1, 2, 3), True), (np.array([1.0, 2.0]), True), (torch.tensor([1.0, 2.0]), True), ("3", True), ({0: 1, 1: 2}, True),
+    ((1,), False), ([], False), (np.array(3.0), False), (torch.tensor(3.0), False), ("ab", False), (None, False)], ids=repr)
+def test_same_ews_radius(monkeypatch, radius, accepted):
+    a, b = _same(monkeypatch, lambda: _call_with(ews_radius=radius))
+    assert a == b and isinstance(a, list) == accepted
+
+
 def test_same_structures_of_both_sides(monkeypatch):
     def call():
         fp.insert_and_extract_central_slices_3d(

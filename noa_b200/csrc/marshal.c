@@ -74,6 +74,25 @@ static int to_int64s(PyObject* seq, int64_t* out, Py_ssize_t count, enum Length 
     return st;
 }
 
+/* Four integers of anything that is read by index: a tuple or a list (the first of a longer one), else by its
+ * own subscripts. */
+static int to_target_shape(PyObject* x, int64_t out[4]) {
+    if (PyTuple_Check(x) || PyList_CheckExact(x))
+        return to_int64s(x, out, 4, HEAD);
+    for (long i = 0; i < 4; ++i) {
+        PyObject* key = PyLong_FromLong(i);
+        PyObject* v = key ? PyObject_GetItem(x, key) : NULL;
+        Py_XDECREF(key);
+        if (!v)
+            return -1;
+        const int st = to_int64(v, &out[i]);
+        Py_DECREF(v);
+        if (st != 0)
+            return -1;
+    }
+    return 0;
+}
+
 /* A tensor, a number (constant input) or None. 1: present, 0: None, -1: error. */
 static int to_array(PyObject* t, nb_array* a) {
     memset(a, 0, sizeof(*a));
@@ -248,7 +267,7 @@ static int to_options(PyObject* o, nb_options* out) {
     if (to_double(PyTuple_GET_ITEM(o, 1), &out->fftfreq_cutoff) != 0)
         return -1;
     PyObject* target = PyTuple_GET_ITEM(o, 2);
-    if (target != Py_None && to_int64s(target, out->target_shape, 4, HEAD) != 0)
+    if (target != Py_None && to_target_shape(target, out->target_shape) != 0)
         return -1;
     if (to_ews_radius(PyTuple_GET_ITEM(o, 3), out->ews_radius) != 0)
         return -1;

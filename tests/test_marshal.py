@@ -90,6 +90,16 @@ def test_same_ews_radius(monkeypatch, radius, accepted):
     assert a == b and isinstance(a, list) == accepted
 
 
+@pytest.mark.parametrize("target,accepted", [
+    (lambda: (1, 8, 8, 8), True), (lambda: [1, 8, 8, 8, 9], True), (lambda: torch.Size((1, 8, 8, 8)), True),
+    (lambda: np.array([1, 8, 8, 8]), True), (lambda: torch.tensor([1, 8, 8, 8, 8]), True), (lambda: {3: 4, 2: 3, 1: 2, 0: 1}, True),
+    (lambda: "1888", True), (lambda: {1: 0, 8: 0, 9: 0, 7: 0}, False), (lambda: (x for x in (1, 8, 8, 8)), False),
+    (lambda: {1, 2, 3, 4}, False), (lambda: (1, 8, 8), False), (lambda: 8, False)])
+def test_same_target_shape(monkeypatch, target, accepted):
+    a, b = _same(monkeypatch, lambda: _call_with(target_shape=target()))
+    assert a == b and isinstance(a, list) == accepted
+
+
 def test_same_structures_of_both_sides(monkeypatch):
     def call():
         fp.insert_and_extract_central_slices_3d(

@@ -25,15 +25,15 @@ static int fail(long code, const char* message) {
     return -1;
 }
 
-/* int(x) and float(x). */
+/* int(x), its low 64 bits as ctypes' integers take it, and float(x). */
 static int to_int64(PyObject* x, int64_t* out) {
     if (PyLong_CheckExact(x)) {
-        *out = PyLong_AsLongLong(x);
+        *out = (int64_t) PyLong_AsUnsignedLongLongMask(x);
     } else {
         PyObject* n = PyNumber_Long(x);
         if (!n)
             return -1;
-        *out = PyLong_AsLongLong(n);
+        *out = (int64_t) PyLong_AsUnsignedLongLongMask(n);
         Py_DECREF(n);
     }
     return *out == -1 && PyErr_Occurred() ? -1 : 0;
@@ -261,8 +261,6 @@ static int to_options(PyObject* o, nb_options* out) {
     int64_t method;
     if (to_int64(interp, &method) != 0)
         return -1;
-    if (method < INT32_MIN || method > INT32_MAX)
-        method = -1; /* not a method: refused by the library */
     out->interp = (int32_t) method;
     if (to_double(PyTuple_GET_ITEM(o, 1), &out->fftfreq_cutoff) != 0)
         return -1;
@@ -315,8 +313,12 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     nb_options options;
     if (to_options(args[8], &options) != 0)
         return NULL;
-    void* stream = args[9] == Py_None ? NULL : PyLong_AsVoidPtr(args[9]);
-    if (PyErr_Occurred())
+    int64_t stream = 0;
+    if (args[9] != Py_None && !PyLong_Check(args[9])) {
+        PyErr_SetString(PyExc_TypeError, "stream: an integer handle is expected");
+        return NULL;
+    }
+    if (args[9] != Py_None && to_int64(args[9], &stream) != 0)
         return NULL;
     PyObject* keep = PyList_New(0);
     if (!keep)
@@ -332,10 +334,10 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     Py_BEGIN_ALLOW_THREADS
     if (n == 12)
         code = ((entry2) entry)((int32_t) remap, present[0], present[1], shapes[0], present[2], present[3], shapes[1],
-                                &xf[0], &xf[1], &options, stream);
+                                &xf[0], &xf[1], &options, (void*) (uintptr_t) stream);
     else
         code = ((entry4) entry)((int32_t) remap, present[0], present[1], shapes[0], present[2], present[3], shapes[1],
-                                &xf[0], &xf[1], &xf[2], &xf[3], &options, stream);
+                                &xf[0], &xf[1], &xf[2], &xf[3], &options, (void*) (uintptr_t) stream);
     Py_END_ALLOW_THREADS
     Py_DECREF(keep);
     return PyLong_FromLong(code);

@@ -100,6 +100,15 @@ def test_same_target_shape(monkeypatch, target, accepted):
     assert a == b and isinstance(a, list) == accepted
 
 
+@pytest.mark.parametrize("big", [2 ** 63, 2 ** 64 + 8, 2 ** 70, -2 ** 63, -2 ** 63 - 1, 2 ** 32 + 1, -1])
+def test_same_integers_beyond_the_structures(monkeypatch, big):
+    def call():
+        fp.extract_central_slices_3d("hc2h", _vol, None, (1, big, 8, 8), _out, None, (3, 1, 8, big), None, _packed,
+                                     stream=big, target_shape=(1, big, 8, 8), interp=big)
+    a, b = _same(monkeypatch, call)
+    assert a == b and isinstance(a, list)
+
+
 def test_same_structures_of_both_sides(monkeypatch):
     def call():
         fp.insert_and_extract_central_slices_3d(

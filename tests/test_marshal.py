@@ -159,3 +159,14 @@ def test_a_module_that_does_not_compile_leaves_the_library_build_going(monkeypat
     monkeypatch.setattr(build.subprocess, "run", lambda *a, **k: subprocess.CompletedProcess(a, 1, "", "no compiler"))
     with pytest.warns(RuntimeWarning, match="no compiler"):
         build._build_marshal()
+
+
+@pytest.mark.parametrize("missing", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_current_stream_without_torchs_private_functions(monkeypatch, missing):
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 11, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 12}))
+    assert fp._stream_ptr(None) == 11
+    monkeypatch.delattr(torch._C, missing)
+    assert fp._stream_ptr(None) == 12

@@ -33,6 +33,21 @@ def test_window_extraction(interp, kw):
     _check(default_case("extract", interp=interp, nslices=3, seed=701, **kw), 1e-5)
 
 
+# A slice whose rotation is NaN: with a w-window every sample passes the cutoff test (it excludes what is
+# larger), so the slice's values and weights are NaN, whatever the interpolation, and the others are not.
+@pytest.mark.parametrize("interp", ["nearest", "linear", "cubic", "cubic_bspline", "lanczos4", "lanczos6", "lanczos8"])
+@pytest.mark.parametrize("dt", ["c32", "f32"])
+def test_nan_rotation_with_w_window(interp, dt):
+    import gpu_run
+    call = build(default_case("extract", interp=interp, n=24, nslices=3, remap="hc2h", in_dt=dt, out_dt=dt, in_w=True,
+                              out_w=True, w_sinc=(0.05, 0.12), seed=709))
+    call.rot[1] = np.nan
+    out, out_w = gpu_run.run(call)
+    if interp != "nearest":  # takes the nearest voxel without weights
+        assert np.isnan(out[1]).all() and np.isnan(out_w[1]).all()
+    assert np.isfinite(out[[0, 2]]).all() and np.isfinite(out_w[[0, 2]]).all()
+
+
 # Run lengths of 1, 2, 4, 8 and 16 rows (148 SMs x 1024 threads decide), the last run of a column shorter.
 @pytest.mark.parametrize("nslices", [7, 400, 800, 1600, 3200])
 def test_rasterize_run_lengths(nslices):

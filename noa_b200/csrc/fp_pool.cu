@@ -104,18 +104,25 @@ void* scratch_alloc(size_t bytes, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         if (!g_pools[dev]) {
+            // A capture's first call may be the first to need the pool. Creating it is no stream operation, but
+            // fails, and breaks the capture, in a thread whose captures are not relaxed.
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.handleTypes = cudaMemHandleTypeNone;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
-            if (cudaMemPoolCreate(&g_pools[dev], &props) != cudaSuccess) {
+            const bool created = cudaMemPoolCreate(&g_pools[dev], &props) == cudaSuccess;
+            uint64_t threshold = UINT64_MAX;
+            if (created)
+                cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &threshold);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (!created) {
                 cudaGetLastError();
                 g_pools[dev] = nullptr;
                 return nullptr;
             }
-            uint64_t threshold = UINT64_MAX;
-            cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &threshold);
         }
         pool = g_pools[dev];
     }

@@ -185,3 +185,46 @@ def test_batch_runs_capture_and_creation_refuses_inside_a_capture():
             ExtractBatch("hc2h", req, interp="linear", autotune=False)
     torch.cuda.synchronize()
     batch.close()
+
+
+_FIRST_CALL = """
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+from noa_b200 import fourier_project as fp, synthetic
+n, count = 64, 200
+vol = torch.from_numpy(synthetic.make_volume(n, seed=1)).cuda()
+rot = fp.pack_rotations(torch.from_numpy(synthetic.random_rotations(count, seed=2)).cuda())
+out = torch.zeros((count, 1, n, n // 2 + 1), dtype=torch.complex64, device="cuda")
+grid = torch.zeros((1, n, n, n // 2 + 1), dtype=torch.complex64, device="cuda")
+
+def step():
+    fp.extract_central_slices_3d("hc2h", vol, None, (1, n, n, n), out, None, (count, 1, n, n), None, rot)
+    fp.rasterize_central_slices_3d("h2hc", out, None, (count, 1, n, n), grid, None, (1, n, n, n), None, rot)
+
+torch.cuda.synchronize()
+side = torch.cuda.Stream()
+side.wait_stream(torch.cuda.current_stream())
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=side):
+    step()
+g.replay()
+torch.cuda.synchronize()
+captured = out.clone(), grid.clone()
+grid.zero_()
+step()
+torch.cuda.synchronize()
+assert torch.equal(captured[0], out) and out.abs().max().item() > 0
+assert ((captured[1] - grid).abs().pow(2).sum() / grid.abs().pow(2).sum()).sqrt().item() <= 1e-6
+print("captured")
+"""
+
+
+def test_a_process_first_call_may_be_captured():
+    """The library's memory pool is made by the first call that needs scratch, here inside a capture."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _FIRST_CALL, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "captured", r.stdout + r.stderr

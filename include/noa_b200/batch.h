@@ -54,12 +54,13 @@ enum { NB_BATCH_AUTOTUNE = 1, NB_BATCH_PERSISTENT_ONLY = 2 };
  * NB_BATCH_AUTOTUNE: by timing the candidates on this batch, once per workload key, cached in memory and
  * in the text file $NB_AUTOTUNE_CACHE or $HOME/.cache/noa_b200/autotune.txt; autotuning runs the batch,
  * so it writes the outputs) and captures the launch into a CUDA graph. Synchronizes `stream`.
- * LINEAR batches over complex volumes (no scaling, EWS, input weights or w-window) hold a pair copy
- * (16 bytes per rfft voxel) of each volume whose requests read enough pixels to pay for it (at least
- * three per voxel), like the per-call entry point; the graph rebuilds these copies at every run, so
+ * LINEAR batches over complex volumes (no input weights or w-window) hold a pair copy (16 bytes per
+ * rfft voxel, rows and planes padded by a few elements) of each volume whose requests read at least two
+ * output pixels per voxel of it (three of a volume of 2^24 voxels and more, for requests run as grids); the graph rebuilds these copies at every run, so
  * changes to the volumes between runs are seen. A LINEAR request with at least 2^16 output pixels runs,
  * in the graph, as a grid of its own (the per-call kernel) on a parallel branch, from its volume or, once
- * it is written, from its volume's copy; the copies are made meanwhile on a higher-priority branch (NB_BATCH_PERSISTENT_ONLY keeps every request in the persistent kernel).
+ * it is written, from its volume's copy; the copies are made meanwhile on a higher-priority branch
+ * (NB_BATCH_PERSISTENT_ONLY keeps every request in the persistent kernel).
  * Results are bit-identical either way. */
 NB_API int nb_extract_batch_create(int32_t remap, const nb_extract_request* requests, int64_t n_requests,
                                    const nb_options* options, int32_t flags, void* stream,

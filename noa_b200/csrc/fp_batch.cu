@@ -440,6 +440,15 @@ using namespace nb;
 
 namespace nb {
 namespace {
+// Pixels per voxel from which a batch holds a pair copy of a volume; BATCH_PAIRS_LARGE for one of twice the L2
+// and more (2^24 voxels) unless the requests that stay in the persistent kernel reach BATCH_PAIRS alone. The
+// per-call rule (pairs_pay) asks for more of small calls, for the copy's allocation, which a batch makes once;
+// without the copies of its volumes a batch's persistent kernel takes the generic instantiation, one pixel per
+// thread, for every request. 4 requests of 2.2 pixels per voxel over 96^3, 192^3 and 384^3 in the persistent kernel: 35,
+// 202 and 1168 us without and 25, 107 and 808 us with copies; over 384^3 as grids of their own 767 and 759 us, 60 requests of
+// 3.2 there 1155 and 1063 us. (The persistent kernel gains from about one pixel per voxel on, 23 and 21 us at 96^3, 115
+// and 70 us at 192^3; the line is at two for the memory that a batch holds and the time to make it.)
+constexpr int64_t BATCH_PAIRS = 2, BATCH_PAIRS_LARGE = 3;
 constexpr size_t NO_JOB = ~size_t(0);  // of a direct request that reads its volume, not a pair copy
 
 // Whether a request gets a grid of its own: LINEAR without a w-window and at least `least` output pixels.
@@ -653,12 +662,12 @@ double time_config(nb_extract_batch_t* h, const Config& c, cudaStream_t stream, 
 }
 
 // LINEAR batches: a pair copy per distinct complex volume whose requests read enough pixels to pay for
-// it (pairs_pay), allocated for the batch's lifetime; without one, or without memory for it, requests
+// it (BATCH_PAIRS), allocated for the batch's lifetime; without one, or without memory for it, requests
 // read the volume. Then the requests that get grids of their own leave the list.
 void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
     if (h->interp != I_LINEAR)
         return;
-    struct Vol { const ProjArgs* a; int64_t pixels; std::vector<size_t> reqs; };
+    struct Vol { const ProjArgs* a; int64_t pixels, persistent; std::vector<size_t> reqs; };
     std::vector<Vol> vols;
     for (size_t i = 0; i < h->host_reqs.size(); ++i) {
         const ProjArgs& a = h->host_reqs[i].a;
@@ -671,15 +680,19 @@ void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
                 c.a->in.s2 == a.in.s2 && c.a->in_centered == a.in_centered)
                 v = &c;
         if (!v) {
-            vols.push_back({&a, 0, {}});
+            vols.push_back({&a, 0, 0, {}});
             v = &vols.back();
         }
-        v->pixels += a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
+        const int64_t pixels = a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
+        v->pixels += pixels;
+        if (!allow_direct || !runs_direct(h->host_reqs[i], DIRECT_MIN_PIXELS))
+            v->persistent += pixels;
         v->reqs.push_back(i);
     }
     for (const Vol& v : vols) {
         const int64_t vox = static_cast<int64_t>(v.a->vol_d) * v.a->vol_h * (v.a->vol_w / 2 + 1);
-        if (!pairs_pay(v.pixels, vox))
+        if (v.pixels < (vox < (int64_t(1) << 24) ? BATCH_PAIRS : BATCH_PAIRS_LARGE) * vox &&
+            v.persistent < BATCH_PAIRS * vox)
             continue;
         ProjArgs copy = *v.a;
         pad_pairs(copy);

@@ -107,6 +107,20 @@ def _per_call_equal(reqs, interp):
         assert torch.equal(r.slice, ref)
 
 
+def _copies(reqs, **kw):
+    """How many pair copies a LINEAR batch of the requests holds: counted by refusing them (the descriptors
+    are smaller than any copy here)."""
+    from noa_b200 import fourier_project as fp
+    from noa_b200.batch import ExtractBatch
+    before = fp.scratch_refusals()
+    fp.set_scratch_limit(1 << 16)
+    try:
+        ExtractBatch("hc2h", reqs, interp="linear", autotune=False, **kw).close()
+    finally:
+        fp.set_scratch_limit(None)
+    return fp.scratch_refusals() - before
+
+
 # Enough items that the persistent kernel claims several consecutive items at a time (more than
 # 2 x 64 per CTA), so runs cross slice and request boundaries inside one claim.
 LARGE = [(128, 1500), (96, 2000), (112, 1201), (64, 903), (128, 700), (80, 1000), (112, 37)]
@@ -191,6 +205,22 @@ def test_linear_batch_pair_copies_follow_volume_updates(tmp_path, monkeypatch):
         v.mul_(-0.5).add_(0.25)
     for r in reqs:
         r.slice.fill_(3)
+    batch.run()
+    torch.cuda.synchronize()
+    _per_call_equal(reqs, "linear")
+    batch.close()
+
+
+@pytest.mark.parametrize("persistent_only", [False, True])
+def test_linear_batch_copies_from_two_pixels_per_voxel(persistent_only):
+    """A batch holds a copy of every volume that its requests read two pixels per voxel of, however few they
+    are and whichever kernel they run in; the same bits as the per-call entry point."""
+    import torch
+    from noa_b200.batch import ExtractBatch
+    reqs, _ = _large_requests([(48, 60), (64, 100), (48, 40), (40, 79), (64, 30), (96, 193)], seed=15)
+    assert _copies(reqs, persistent_only=persistent_only) == 3  # 48 (100 slices), 64 (130) and 96; not 40 (79)
+    batch = ExtractBatch("hc2h", reqs, interp="linear", autotune=False, persistent_only=persistent_only)
+    assert (batch.info()["n_direct"] > 0) != persistent_only
     batch.run()
     torch.cuda.synchronize()
     _per_call_equal(reqs, "linear")

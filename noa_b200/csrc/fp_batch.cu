@@ -162,9 +162,11 @@ template<int I, bool WINDOW = has_window<I>()> struct BatchSlots { using T = Win
 template<int I> struct BatchSlots<I, false> { struct T {}; };
 
 // PAIRS_ONLY: every request reads a pair copy (LINEAR, complex); the generic path is compiled out so
-// the kernel fits 48 registers (5 CTAs per SM, like extract_linear_kernel).
+// the kernel fits 48 registers (5 CTAs per SM, like extract_linear_kernel; with six the persistent launch is
+// 2 to 18 % slower at 64^3 to 256^3, 60 requests of 256^3 379 and 420 us, and 1 to 3 % faster for a few requests
+// of 384^3). The generic LINEAR kernel keeps three (the compiler's 94 registers leave two: a quarter slower).
 template<int I, bool IN_C, bool OUT_C, int V, bool PAIRS_ONLY = false>
-__global__ void __launch_bounds__(256, PAIRS_ONLY ? 5 : VARIANTS[V].min_ctas)
+__global__ void __launch_bounds__(256, PAIRS_ONLY ? 5 : I == I_LINEAR && VARIANTS[V].min_ctas < 3 ? 3 : VARIANTS[V].min_ctas)
 batch_extract_kernel(const BatchReq* __restrict__ reqs, int n_req, int64_t n_items,
                      unsigned long long* __restrict__ counter) {
     constexpr Variant VT = VARIANTS[V];

@@ -26,10 +26,10 @@ namespace {
 constexpr int TY = 16, TX = 16, EXTRACT_THREADS = TY * TX;
 
 // ---------------------------------------------------------------------------------------------------
-// Fast LINEAR path over a pair copy of the volume (fp_pairs.cuh). Each thread interpolates PAIR_PPT
+// Fast LINEAR path over a pair copy of the volume (fp_pairs.cuh). Each thread interpolates PPT
 // pixels (rows y, y+16, ...) of one column, keeping more loads in flight.
 // ---------------------------------------------------------------------------------------------------
-constexpr int PAIR_PPT = 4;
+constexpr int PPT = 4;
 
 // The w-window's offsets and values do not depend on the pixel, so a CTA tabulates them once (the same
 // expressions as the per-sample ones, hence the same bits) instead of dividing and evaluating the window
@@ -71,7 +71,7 @@ __global__ void make_pairs(const __grid_constant__ ProjArgs a, float4* __restric
 // from the volume (eight loads). Same bits
 // as one slice per CTA and one pixel at a time: 4096 slices of 256^3 1195 us -> 1164 us with the copy
 // (1104 us with the copy padded, pad_pairs); 150 slices of 200^3 without it 50.1 us -> 41.2 us.
-template<bool PAIRS, bool IN_C, bool OUT_C, int PPT, typename Idx>
+template<bool PAIRS, bool IN_C, bool OUT_C, typename Idx>
 __global__ void __launch_bounds__(EXTRACT_THREADS, 5)
 extract_linear_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx, int per_cta,
                       bool lanes_16) {
@@ -150,7 +150,7 @@ int slices_per_cta(int64_t tiles, int64_t slices) {
     return static_cast<int>(s < 1 ? 1 : s > 8 ? 8 : s);
 }
 
-template<bool PAIRS, bool IN_C, bool OUT_C, int PPT, typename Idx>
+template<bool PAIRS, bool IN_C, bool OUT_C, typename Idx>
 cudaError_t launch_linear(const ProjArgs& a, const float4* pairs, cudaStream_t stream) {
     const int wp = a.slice_w / 2 + 1;
     const int ntx = (wp + TX - 1) / TX, nty = (a.slice_h + TY * PPT - 1) / (TY * PPT);
@@ -161,18 +161,20 @@ cudaError_t launch_linear(const ProjArgs& a, const float4* pairs, cudaStream_t s
     // all start on the same banks (boxes that are a multiple of 32) are read with 3.4 lines a group by lanes
     // in a row and 4.1 by lanes in two rows of 8, others with 2.5 and 2.3 (replayed on the CPU).
     const bool lanes_16 = !PAIRS && a.in.s0 % 16 == 0;
-    extract_linear_kernel<PAIRS, IN_C, OUT_C, PPT, Idx><<<grid, EXTRACT_THREADS, 0, stream>>>(a, pairs, ntx, per_cta, lanes_16);
+    extract_linear_kernel<PAIRS, IN_C, OUT_C, Idx><<<grid, EXTRACT_THREADS, 0, stream>>>(a, pairs, ntx, per_cta, lanes_16);
     return cudaGetLastError();
 }
 
-// Without a pair copy: four pixels per thread once one pixel per thread would be two rounds of the chip's
-// 2048 threads per SM.
-template<bool IN_C, bool OUT_C, typename Idx>
-cudaError_t launch_linear_volume(const ProjArgs& a, cudaStream_t stream) {
+// Without a pair copy: whether the launch is large enough for four pixels per thread. One pixel per thread
+// (extract_kernel) has four times the threads to hide the taps' latency with, up to so many rounds of the chip's
+// 2048 threads per SM (303 k pixels): five for complex values, six with input weights, four for real values. us of
+// extract_kernel and of extract_linear_kernel, means over boxes of 48 to 256: 0.65 M pixels 12.5 and 14.1, 1.3 M 21.9 and
+// 21.9, 1.8 M 28.8 and 27.5; with weights 1.3 M 31.3 and 33.5, 1.8 M 41.4 and 41.8; real 0.65 M 11.4 and 12.1, 0.9 M 14.8
+// and 15.2, 1.3 M 20.0 and 19.0.
+bool use_linear_kernel(const ProjArgs& a) {
     const int64_t pixels = a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
-    if (pixels >= static_cast<int64_t>(sm_count()) * 4096)
-        return launch_linear<false, IN_C, OUT_C, PAIR_PPT, Idx>(a, nullptr, stream);
-    return launch_linear<false, IN_C, OUT_C, 1, Idx>(a, nullptr, stream);
+    const int rounds = !a.in_cplx ? 4 : a.in_w.present && a.out_w.present ? 6 : 5;
+    return a.interp == I_LINEAR && a.wsize <= 1 && pixels >= static_cast<int64_t>(sm_count()) * 2048 * rounds;
 }
 
 // The w-windowed form over the pair copy: per pixel, the windowed sum over the w offsets of the
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(EXTRACT_THREADS)
 extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restrict__ pairs, int ntx) {
     const int wp = a.slice_w / 2 + 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y0 = (blockIdx.x / ntx) * (TY * PAIR_PPT) + (warp >> 1) * 4 + pair_row(lane);
+    const int y0 = (blockIdx.x / ntx) * (TY * PPT) + (warp >> 1) * 4 + pair_row(lane);
     const int u = (blockIdx.x % ntx) * TX + (warp & 1) * 8 + pair_column(lane);
     __shared__ float2 s_w[W_TABLE];
     fill_w_table(a, s_w);
@@ -201,7 +203,7 @@ extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restr
 
     for (int64_t b = blockIdx.y; b < a.n_slices; b += gridDim.y) {
 #pragma unroll 1
-        for (int r = 0; r < PAIR_PPT; ++r) {
+        for (int r = 0; r < PPT; ++r) {
             const int y = y0 + r * TY;
             if (y >= a.slice_h)
                 break;
@@ -252,12 +254,14 @@ extract_pairs_w_kernel(const __grid_constant__ ProjArgs a, const float4* __restr
 
 // Whether the per-call pair path applies: the pair copy is readable (pairs_apply) and there are enough
 // pixels to amortise making it.
-bool use_pairs(const ProjArgs& a) {
+bool use_pairs(const ProjArgs& a, cudaStream_t stream) {
     const int64_t vox = static_cast<int64_t>(a.vol_d) * a.vol_h * (a.vol_w / 2 + 1);
     const int64_t pix = a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
     ProjArgs plain = a;
     plain.wsize = 1;  // the w-windowed form reads the pair copy too (extract_pairs_w_kernel)
-    return pairs_apply(plain) && pairs_pay(pix * (a.wsize > 1 ? a.wsize : 1), vox);
+    if (!pairs_apply(plain))
+        return false;
+    return a.wsize > 1 ? pairs_pay_w(pix * a.wsize, vox) : pairs_pay(pix, vox, stream);
 }
 
 cudaError_t launch_pairs(const ProjArgs& call, cudaStream_t stream, bool& done) {
@@ -274,7 +278,7 @@ cudaError_t launch_pairs(const ProjArgs& call, cudaStream_t stream, bool& done) 
     return err;
 }
 
-// NEAREST, and LINEAR with a w-window where the pair copy does not apply: one pixel per thread.
+// NEAREST, and LINEAR from the volume in small launches or with a w-window: one pixel per thread.
 template<int I, bool IN_C, bool OUT_C, typename Idx>
 __global__ void __launch_bounds__(EXTRACT_THREADS)
 extract_kernel(const __grid_constant__ ProjArgs a, int ntx) {
@@ -355,9 +359,11 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
     if (a.n_slices == 0)
         return cudaSuccess;
     const dim3 grid(static_cast<unsigned>(ntx * nty), static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
-    if (I == I_LINEAR && a.wsize <= 1)
-        return a.wide_in ? launch_linear_volume<IN_C, OUT_C, int64_t>(a, stream)
-                         : launch_linear_volume<IN_C, OUT_C, int32_t>(a, stream);
+    if constexpr (I == I_LINEAR) {
+        if (use_linear_kernel(a))
+            return a.wide_in ? launch_linear<false, IN_C, OUT_C, int64_t>(a, nullptr, stream)
+                             : launch_linear<false, IN_C, OUT_C, int32_t>(a, nullptr, stream);
+    }
     if constexpr (has_window<I>()) {
         if (a.in_bytes_narrow)
             extract_window_kernel<I, IN_C, OUT_C, uint32_t><<<grid, EXTRACT_THREADS, 0, stream>>>(a, ntx);
@@ -387,10 +393,10 @@ cudaError_t launch_extract_pairs(const ProjArgs& a, const float4* pairs, cudaStr
     if (a.n_slices <= 0)
         return cudaSuccess;
     if (a.wsize <= 1)
-        return a.out_cplx ? launch_linear<true, true, true, PAIR_PPT, int>(a, pairs, stream)
-                          : launch_linear<true, true, false, PAIR_PPT, int>(a, pairs, stream);
+        return a.out_cplx ? launch_linear<true, true, true, int>(a, pairs, stream)
+                          : launch_linear<true, true, false, int>(a, pairs, stream);
     const int wp = a.slice_w / 2 + 1;
-    const int ntx = (wp + TX - 1) / TX, nty = (a.slice_h + TY * PAIR_PPT - 1) / (TY * PAIR_PPT);
+    const int ntx = (wp + TX - 1) / TX, nty = (a.slice_h + TY * PPT - 1) / (TY * PPT);
     const dim3 grid(static_cast<unsigned>(ntx * nty), static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
     if (a.out_cplx)
         extract_pairs_w_kernel<true><<<grid, EXTRACT_THREADS, 0, stream>>>(a, pairs, ntx);
@@ -425,7 +431,7 @@ cudaError_t launch_make_pairs(const ProjArgs& a, float4* pairs, cudaStream_t str
 cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream) { return launch_interp<I_LINEAR>(a, stream); }
 
 cudaError_t launch_extract(const ProjArgs& a, cudaStream_t stream) {
-    if (a.n_slices > 0 && use_pairs(a)) {
+    if (a.n_slices > 0 && use_pairs(a, stream)) {
         bool done = false;
         const cudaError_t err = launch_pairs(a, stream, done);
         if (err != cudaSuccess || done)

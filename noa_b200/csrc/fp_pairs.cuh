@@ -7,6 +7,7 @@
 #pragma once
 
 #include "fp_args.cuh"
+#include "fp_pool.cuh"
 
 namespace nb {
 
@@ -188,13 +189,22 @@ inline bool pairs_apply(const ProjArgs& a) {
            vox < (int64_t(1) << 31);
 }
 
-// From how many output pixels on a LINEAR extraction is faster through a pair copy made for it: three per
-// voxel, four where the copy is twice the L2 and more (2^24 voxels), and 2 M. Measured without and with, us:
-// 64^3 x 256 slices (4 pixels per voxel) 15 and 17; 128^3 x 256 (2) 34 and 35, x 384 (3) 45 and 41; 200^3 x 400 (2)
-// 93 and 101, x 600 (3) 135 and 129; 256^3 x 512 (2) 196 and 196, x 768 (3) 276 and 243; 384^3 x 1152 (3) 959 and
-// 962, x 1536 (4) 1328 and 1253; 512^3 x 1536 (3) 2489 and 2622, x 2048 (4) 3349 and 3390, x 4096 (8) 6778 and 6473.
-inline bool pairs_pay(int64_t pixels, int64_t voxels) {
-    return pixels >= (voxels < (int64_t(1) << 24) ? 3 : 4) * voxels && pixels >= (int64_t(1) << 21);
+// From how many output pixels on a LINEAR extraction is faster through a pair copy made for it: two per
+// voxel, four where the copy is twice the L2 and more (2^24 voxels), and 3 * 2^19 for its allocation and launch;
+// 3 * 2^17 in a stream capture, where the allocation is a node of the graph. Called one after another, us without and
+// with: 64^3 x 384 slices (6 pixels per voxel) 18 and 19, x 512 (8) 21 and 20; 96^3 x 192 (2) 21 and 21, x 384 (4) 31 and 29;
+// 128^3 x 192 (1.5) 28 and 27, x 256 (2) 33 and 31, x 512 (4) 57 and 48; 160^3 x 320 (2) 58 and 51; 256^3 x 512 (2) 196 and 187,
+// x 768 (3) 276 and 243; 384^3 x 1152 (3) 959 and 962, x 1536 (4) 1328 and 1253; 512^3 x 1536 (3) 2489 and 2622, x 2048 (4) 3349 and
+// 3390, x 4096 (8) 6778 and 6473. In a graph: 64^3 x 160 (2.5) 9.1 and 9.1, x 192 (3) 10.6 and 9.0; 96^3 x 192 (2) 19 and 16;
+// 128^3 x 256 (2) 32 and 26; 384^3 x 960 (2.5) 812 and 823.
+inline bool pairs_pay(int64_t pixels, int64_t voxels, cudaStream_t stream) {
+    return pixels >= (voxels < (int64_t(1) << 24) ? 2 : 4) * voxels && pixels >= 3 * (int64_t(1) << 17) &&
+           (pixels >= 3 * (int64_t(1) << 19) || stream_capturing(stream));
+}
+
+// The same of the w-windowed extraction, by samples: three per voxel (four), and 2 M.
+inline bool pairs_pay_w(int64_t samples, int64_t voxels) {
+    return samples >= (voxels < (int64_t(1) << 24) ? 3 : 4) * voxels && samples >= (int64_t(1) << 21);
 }
 
 // The per-call LINEAR extraction from the volume itself (no w-window).
@@ -204,8 +214,8 @@ cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream);
 // `priority`, the launch carries that scheduling priority (kept by a graph captured from it).
 cudaError_t launch_make_pairs(const ProjArgs& a, float4* pairs, cudaStream_t stream, const int* priority = nullptr);
 
-// The per-call LINEAR extraction over a pair copy of a.in: one grid of (slice tile, slice) CTAs
-// (extract_pairs_kernel, or extract_pairs_w_kernel with a w-window).
+// The per-call LINEAR extraction over a pair copy of a.in: one grid of (slice tile, slices) CTAs
+// (extract_linear_kernel, or extract_pairs_w_kernel with a w-window).
 cudaError_t launch_extract_pairs(const ProjArgs& a, const float4* pairs, cudaStream_t stream);
 
 } // namespace nb

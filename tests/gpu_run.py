@@ -22,6 +22,18 @@ def _xform(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
+def scratch_wanted(fn):
+    """How many allocations of its own the library asks for in ``fn()``, counted by refusing them all, and
+    what ``fn`` returns on the paths that calls take without. An extraction asks for its pair copy alone."""
+    before = fp.scratch_refusals()
+    fp.set_scratch_limit(0)
+    try:
+        result = fn()
+    finally:
+        fp.set_scratch_limit(None)
+    return fp.scratch_refusals() - before, result
+
+
 def run(call: Call, stream=None, scatter=False):
     """Copies the call's inputs to the device, runs the CUDA path, returns (out, out_w) as numpy.
     ``scatter``: insertions run the slice-major scatter form instead of the gather form."""

@@ -9,9 +9,12 @@ from oracle.oracle import FpOracle
 pytestmark = pytest.mark.gpu
 
 
-def _check(case, tol, **kw):
+def _check(case, tol, copies=None, **kw):
+    """`copies`: how many pair copies the call has to make (None: not looked at)."""
     import gpu_run
     call = build(case)
+    if copies is not None:
+        assert gpu_run.scratch_wanted(lambda: gpu_run.run(clone(call), **kw))[0] == copies
     ref = clone(call)
     assert FpOracle().run(ref, 8) == 0
     out, out_w = gpu_run.run(clone(call), **kw)
@@ -89,14 +92,24 @@ def test_pair_queue(kw):
 
 
 # LINEAR extraction: several slices per CTA with a shorter last group, rows past the slice, cells at the
-# edges of the volume and the non-centered wrap, with and without the pair copy.
+# edges of the volume and the non-centered wrap; over a pair copy, from the volume with four pixels per thread
+# (1.52 M pixels, 1.82 M with input weights, 1.22 M real) and with one.
 @pytest.mark.parametrize("remap", ["h2h", "hc2hc"])
-@pytest.mark.parametrize("kw", [dict(n=20, nslices=1030), dict(n=21, slice_n=70, nslices=513, target=(1, 70, 70, 70), cutoff=0.9),
-                                dict(n=64, nslices=301, in_w=True, out_w=True), dict(n=40, nslices=800, out_dt="f32", out_w=True),
-                                dict(n=40, nslices=800, in_dt="f32", out_dt="f32")],
-                         ids=["pairs", "beyond", "weights", "power", "real"])
-def test_linear_extraction_groups(kw, remap):
-    _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5)
+@pytest.mark.parametrize("copies,kw", [(1, dict(n=20, nslices=9700)), (0, dict(n=20, nslices=1030)),
+                                       (1, dict(n=21, slice_n=70, nslices=841, target=(1, 70, 70, 70), cutoff=0.9)),
+                                       (0, dict(n=21, slice_n=70, nslices=610, target=(1, 70, 70, 70), cutoff=0.9)),
+                                       (0, dict(n=21, slice_n=70, nslices=513, target=(1, 70, 70, 70), cutoff=0.9)),
+                                       (1, dict(n=40, nslices=2600, out_dt="f32", out_w=True)),
+                                       (0, dict(n=40, nslices=1830, out_dt="f32", out_w=True)),
+                                       (0, dict(n=40, nslices=800, out_dt="f32", out_w=True)),
+                                       (0, dict(n=64, nslices=870, in_w=True, out_w=True)),
+                                       (0, dict(n=64, nslices=301, in_w=True, out_w=True)),
+                                       (0, dict(n=40, nslices=1450, in_dt="f32", out_dt="f32")),
+                                       (0, dict(n=40, nslices=800, in_dt="f32", out_dt="f32"))],
+                         ids=["pairs", "small", "beyond-pairs", "beyond", "beyond-small", "power-pairs", "power", "power-small",
+                              "weights", "weights-small", "real", "real-small"])
+def test_linear_extraction_groups(kw, copies, remap):
+    _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5, copies)
 
 
 # The rule on making a pair copy (three pixels per voxel, 2 M pixels), its padded strides, and requests of a

@@ -37,10 +37,12 @@ def _capture(fn):
     return g
 
 
-def test_extract_and_rasterize_replay_equals_eager():
+@pytest.mark.parametrize("count", [200, 1000])
+def test_extract_and_rasterize_replay_equals_eager(count):
+    import gpu_run
     import torch
     from noa_b200 import fourier_project as fp
-    n, count = 64, 200  # enough pixels for the pair copy (200 x 64 x 33 > 2 x 64 x 64 x 33)
+    n = 64  # 1000 slices are enough pixels for the pair copy, 200 only in a capture (3 * 2^19 and 3 * 2^17)
     vol, rot = _inputs(n, count, seed=1)
     vshape, sshape = (1, n, n, n), (count, 1, n, n)
     out = torch.empty((count, 1, n, n // 2 + 1), dtype=torch.complex64, device="cuda")
@@ -51,6 +53,8 @@ def test_extract_and_rasterize_replay_equals_eager():
         fp.extract_central_slices_3d("hc2h", vol, None, vshape, out, None, sshape, None, rot)
         fp.rasterize_central_slices_3d("h2hc", out, None, sshape, grid, grid_w, vshape, None, rot)
 
+    assert gpu_run.scratch_wanted(lambda: fp.extract_central_slices_3d("hc2h", vol, None, vshape, out, None, sshape, None,
+                                                                       rot))[0] == (count == 1000)
     step()
     torch.cuda.synchronize()
     ref_out, ref_grid, ref_w = out.clone(), grid.clone(), grid_w.clone()

@@ -376,8 +376,19 @@ cudaError_t launch_linear(const ProjArgs& a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// Whether insert_linear_kernel applies.
+// Whether insert_linear_kernel applies, and pays: with a quarter of the threads it needs many bricks to fill the
+// chip, and the slices through the brick at the origin, one after another, take it longer (1.15 us each against
+// 0.67 us), so a launch has to hold 320 bricks for one slice, more for more slices, up to 12,000, from where on the
+// other bricks' work outlasts that one. us of the general kernel and of this one, half-width 1 (6), with weights:
+// one slice into 48^3 7.1 and 8.4, 80^3 11.6 and 8.7; 8 into 96^3 18 and 17 (21 and 18); 50 into 128^3 60 and 69 (74 and
+// 76), 160^3 78 and 77 (106 and 88); 400 into 64^3 273 and 450, 176^3 441 and 538 (605 and 625), 224^3 613 and 635 (961
+// and 770), 256^3 889 and 698 (1421 and 877).
 bool use_linear(const ProjArgs& a) {
+    const double bricks = static_cast<double>((a.vol_d + LIN_Z - 1) / LIN_Z) * ((a.vol_h + LIN_Y - 1) / LIN_Y) *
+                          ((a.vol_w / 2 + LIN_X) / LIN_X);
+    const double slices = static_cast<double>(a.n_slices);
+    if (bricks < 12000. && bricks * bricks * bricks < 320. * 320. * 320. * slices * slices)
+        return false;
     return linear_slices(a) && a.rot.kind == 2 && a.scale.kind == 0 && !a.ews.on && a.n_slices < (int64_t(1) << 31);
 }
 

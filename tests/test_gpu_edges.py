@@ -79,6 +79,25 @@ def test_linear_insertion(kw, scatter):
     _check(default_case("insert", **{"seed": 704, **kw}), 1e-5, scatter=scatter)
 
 
+# The same for the gather form by packed pairs of voxels, which takes launches of many 8^3 bricks: 320 for one
+# slice, 320 s^(2/3) for s, 12,000 for any number. Its smallest launches, partly filled bricks on every
+# axis, a second pass of the list (256 slices each), and the other options as above; and the general
+# kernel just below each line.
+@pytest.mark.parametrize("linear,kw", [
+    (True, dict(n=64, nslices=1, out_w=True)), (False, dict(n=56, nslices=1, out_w=True)),
+    (True, dict(n=85, nslices=3, slice_n=70, in_w=True, out_w=True, remap="h2hc", cutoff=0.8)),
+    (False, dict(n=72, nslices=3, slice_n=70, in_w=True, out_w=True, remap="h2hc", cutoff=0.8)),
+    (True, dict(n=84, nslices=3, in_dt="f32", out_dt="f32", in_w=True, out_w=True, sinc=(-1.0, 1.5))),
+    (True, dict(n=97, nslices=4, in_dt="c32", out_dt="f32", remap="h2h", sinc=(-1.0, 0.2))),
+    (True, dict(n=131, nslices=17, sinc=(0.01, 6 / 131), remap="hc2hc")),
+    (True, dict(n=227, nslices=260, remap="hc2hc")), (False, dict(n=217, nslices=260, remap="hc2hc"))],
+    ids=["one", "one-below", "weights", "weights-below", "real", "power", "wide", "passes", "passes-below"])
+def test_linear_insertion_kernel(linear, kw):
+    bricks = ((kw["n"] + 7) // 8) ** 2 * ((kw["n"] // 2 + 8) // 8)
+    assert linear == (bricks >= 12000 or bricks ** 3 >= 320 ** 3 * kw["nslices"] ** 2)
+    _check(default_case("insert", **{"seed": 707, **kw}), 1e-5)
+
+
 # The pair queue: fewer pairs than a half, halves that fill exactly and by many slices, a second pass of the
 # input slices (4096 each), the general rotation, windows over the whole slice, w offsets.
 @pytest.mark.parametrize("kw", [dict(n=12, nslices=1, nout=2), dict(n=10, nslices=4200, nout=1, out_w=True),

@@ -46,10 +46,11 @@ __device__ __forceinline__ void acc_red(void* acc, int off, float2 v, float w) {
 }
 
 // Six CTAs per SM for the LINEAR and NEAREST instantiations (39 registers, no spills): 512^3 x 20,000
-// slices, 378.6 -> 364.2-365.1 ms on one box (1000 slices: 19.32 -> 18.79-18.82 ms). The wider windows
-// keep the compiler's choice.
+// slices, 378.6 -> 364.2-365.1 ms on one box (1000 slices: 19.32 -> 18.79-18.82 ms). Left to the compiler the
+// wider windows take up to 96 registers (two CTAs): 400 slices into 256^3, CUBIC 2280 us and 1440 us with four CTAs asked
+// for; LANCZOS6 4640 us and 3280 us, LANCZOS8 8070 us and 6430 us with three.
 template<int I>
-constexpr int scatter_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 6 : 1; }
+constexpr int scatter_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 6 : I == I_CUBIC || I == I_BSPLINE ? 4 : 3; }
 
 template<int I, bool IN_C, bool W>
 __global__ void __launch_bounds__(SCATTER_THREADS, scatter_min_ctas<I>())

@@ -8,20 +8,22 @@
 // meets the slab are compacted, in increasing order, into shared memory, 4096 at a time, each warp
 // compacting its own range of slice indices so that building the list needs no barrier.
 //
-// Each warp then takes the list 32 slices at a time, one per lane, with no barrier until the next pass. fz is
+// Each warp then takes the list 32 slices at a time, one per lane, with no barrier until the next pass. Where
+// slabs are about as thick as a patch is wide, or few slices meet a patch, it culls them over its own box and
+// walks the rest, every lane evaluating its own pixel of one slice (WALK). Where they are thinner, that leaves half
+// of the lanes idle (17 of 32 active with the default window), and it goes by a queue: fz is
 // linear along a row of pixels, so a slice's slab covers an interval of each of the warp's four rows
 // (widened by the rounding of the exact test): together a 32-bit mask of pixels. The warp walks the slices
 // whose mask is not empty, queues their (pixel, slice) pairs and evaluates queued pairs 64 at a time, two per
-// lane, whichever pixels they belong to: exact distance, window and interpolation run with all lanes busy,
-// although a third of the pixels lie within any one slice's slab. Each lane keeps the queue slots of its own
-// pixel's pairs as a bit mask and adds their results in slot order. (Every lane evaluating its own pixel of
-// one slice at a time had 17 of 32 lanes active; masks transposed so that each lane walks its own pixel's
-// slices without a queue were 10 % slower, the longest list of 32 setting the pace.)
+// lane, whichever pixels they belong to: exact distance, window and interpolation run with all lanes busy.
+// Each lane keeps the queue slots of its own pixel's pairs as a bit mask and adds their results in slot order.
+// (Masks transposed so that each lane walks its own pixel's slices without a queue were 10 % slower, the
+// longest list of 32 setting the pace.)
 //
 // The slices through a pixel grow as 1 / |f|, so the tiles around the origin hold up to 20 times the pairs
-// of the others, and the warp at the origin works for a good part of the launch: tiles are taken in the order
-// of their distance to it, those of all output slices together, so that the long ones start first. 2000
-// input to 64 output slices of 256^2, default window and weights: 3180 us ->
+// of the others, and the warp at the origin works for a good part of the launch: in launches of several tiles
+// per SM, tiles are taken in the order of their distance to it, those of all output slices together, so that the
+// long ones start first. 2000 input to 64 output slices of 256^2, default window and weights: 3180 us ->
 // 1837 us with a queue filled by exact tests and evaluated 32 pairs at a time -> 1253 us.
 //
 // Summation order per pixel is therefore the reference's (increasing slice index). With an Ewald
@@ -95,41 +97,80 @@ struct PairQueue {
     float weight[IE_HALF];
 };
 
-// Whether the pairs take the short arithmetic: Mat33 rotations without scaling or curvature and, for
-// LINEAR, slices that LinearCell can read.
-template<int I>
-bool use_lean(const ProjArgs& a) {
-    return a.rot.kind == 2 && a.scale.kind == 0 && !a.ews.on && (I != I_LINEAR || linear_slices(a));
-}
+// How a warp evaluates the pairs of a slice (form_of chooses).
+enum Form {
+    WALK,   // every lane evaluates its own pixel, one slice at a time
+    QUEUE,  // by the queue, one pair per lane at a time
+    LEAN,   // by the queue, for Mat33 rotations without scaling: LINEAR two pairs per lane in packed operations
+};
 
-template<int I>
-constexpr int insert_extract_min_ctas() { return I == I_LINEAR || I == I_NEAREST ? 4 : 1; }
+// Resident CTAs per SM asked of the compiler. WALK: 5 (48 registers; with 6 3 % slower for quaternions and scaling,
+// equal for matrices). The wider windows: 2, where the compiler's choice for the queue was one, up to 1.4 times
+// slower.
+template<int I, Form FORM>
+constexpr int insert_extract_min_ctas() { return I != I_LINEAR && I != I_NEAREST ? 2 : FORM == WALK ? 5 : 4; }
 
-template<int I, bool IN_C, bool OUT_C, bool LEAN, typename Idx = int>
-__global__ void __launch_bounds__(IE_THREADS, insert_extract_min_ctas<I>())
-insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per_slice, int64_t n_tiles) {
+template<int I, bool IN_C, bool OUT_C, Form FORM, typename Idx = int>
+__global__ void __launch_bounds__(IE_THREADS, insert_extract_min_ctas<I, FORM>())
+insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int nty, int64_t n_tiles, bool by_place) {
     __shared__ int s_list[IE_LIST];
     __shared__ int s_warp_count[IE_THREADS / 32];
     __shared__ float s_box[4][IE_THREADS / 32];
-    __shared__ PairQueue s_queue[IE_THREADS / 32];
+    __shared__ PairQueue s_queue[FORM == WALK ? 1 : IE_THREADS / 32];
 
     const int wp = a.slice_w / 2 + 1;
     const Spectrum2 sp{a.in_h, a.in_w_, a.in_centered, a.in_slice_narrow != 0};
     const bool has_out_w = a.out_w.present;
     const bool has_in_w = a.in_w.present;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    PairQueue& queue = s_queue[warp];
+    PairQueue& queue = s_queue[FORM == WALK ? 0 : warp];
     const WindowPair window_of(a);
+    const bool mat33 = a.rot.kind == 2 && a.scale.kind == 0 && !a.ews.on;
+
+    // Where the sample (z, y, x) lies relative to input slice i: its distance and in-slice frequencies.
+    const auto locate = [&](int64_t i, float z, float y, float x, float& q0, float& q1) {
+        float f0, f1, fz;
+        if (FORM == LEAN || mat33) {
+            // grid2slice's Mat33 rows (same products and sums)
+            const float* m = xform_ptr(a.rot, i, 12);
+            fz = dot3(m[0], m[1], m[2], z, y, x);
+            if (FORM == WALK && !(fabsf(fz) < a.fb))
+                return fz;  // the in-plane rows are only needed inside the slab
+            f0 = dot3(m[3], m[4], m[5], z, y, x);
+            f1 = dot3(m[6], m[7], m[8], z, y, x);
+        } else {
+            fz = grid2slice(z, y, x, a.scale, a.rot, i, a.ews, f0, f1);
+        }
+        q0 = mul(f0, a.f_in0);
+        q1 = mul(f1, a.f_in1);
+        return fz;
+    };
+    // The term of input slice i there, inside its slab.
+    const auto term = [&](int64_t i, float fz, float q0, float q1, float2& value, float& weight) {
+        weight = windowed_sinc_fast(fz, a.pfs, a.ifs, a.pfb);
+        value = cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, i, q0, q1), weight);
+        if (has_in_w)
+            weight = mul(interp_spectrum_2d<I, false>(a.in_w, sp, i, q0, q1).x, weight);
+    };
 
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        // The tile's place by distance to the origin (column of tiles, then rows alternately below and above
-        // the origin's), all output slices of one place together.
-        const int place = static_cast<int>(tile / a.n_slices);
-        const int64_t b = tile - place * a.n_slices;
-        const int nty = tiles_per_slice / ntx;
-        const int tx = place / nty, k_row = place - tx * nty;
-        const int origin = a.out_centered ? a.slice_h / 2 / IE_TILE : 0;
-        const int ty = (origin + (k_row & 1 ? nty - (k_row + 1) / 2 : k_row / 2)) % nty;
+        // by_place: the tile's place by distance to the origin (column of tiles, then rows alternately below and
+        // above the origin's), all output slices of one place together.
+        int64_t b;
+        int tx, ty;
+        if (by_place) {
+            const int place = static_cast<int>(tile / a.n_slices);
+            b = tile - place * a.n_slices;
+            tx = place / nty;
+            const int k_row = place - tx * nty;
+            ty = (a.out_centered ? a.slice_h / 2 / IE_TILE : 0) + (k_row & 1 ? nty - (k_row + 1) / 2 : k_row / 2);
+            ty -= ty < nty ? 0 : nty;
+        } else {
+            b = tile / (ntx * nty);
+            const int t = static_cast<int>(tile - b * (ntx * nty));
+            ty = t / ntx;
+            tx = t - ty * ntx;
+        }
         const int py = ty * IE_TILE + (warp >> 1) * 4 + (lane >> 3);
         const int pu = tx * IE_TILE + (warp & 1) * 8 + (lane & 7);
         const bool valid = py < a.slice_h && pu < wp;
@@ -160,12 +201,16 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
             }
         }
         const bool warp_valid = __any_sync(0xffffffffu, valid);
+        const Box2 wbox = Box2::of(bmin[0], bmax[0], bmin[1], bmax[1]);  // every lane holds its warp's
         // The warp's rows and columns (the non-centered layout wraps between rows, not along them).
-        float rows[4];
+        float rows[4] = {}, step = 0.f, first = 0.f;
+        if constexpr (FORM != WALK) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            rows[r] = __shfl_sync(0xffffffffu, pf0, 8 * r);
-        const float first = __shfl_sync(0xffffffffu, static_cast<float>(pu), 0) / a.f_slice1;
+            for (int r = 0; r < 4; ++r)
+                rows[r] = __shfl_sync(0xffffffffu, pf0, 8 * r);
+            step = 1.f / a.f_slice1;
+            first = __shfl_sync(0xffffffffu, static_cast<float>(pu), 0) * step;
+        }
         __syncthreads();
         float lo[2], hi[2];
 #pragma unroll
@@ -216,74 +261,81 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
 
                 int filled = 0;                           // queued pairs, counted from the pass' start
                 unsigned long long mine0 = 0, mine1 = 0;  // this lane's pixel's slots of the ring's two halves
-                // Evaluates `n` pairs of a half, two per lane, and adds each pixel's.
+                // Evaluates `n` pairs of a half and adds each pixel's.
                 auto evaluate = [&](int half, int n) {
                     __syncwarp();
-                    int64_t si[2];
-                    float q0[2], q1[2], fz[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
+                    // Pair lane + 32 e of the half; past n the first one, outside every slab.
+                    const auto prepare = [&](int e, int64_t& i, float& q0, float& q1) {
                         const int at = lane + 32 * e;
-                        // past n: stale, read as the first pair and not stored
                         const unsigned entry = queue.entry[half * IE_HALF + (at < n ? at : 0)];
                         const int owner = static_cast<int>(entry & 31u);
                         const float z = __shfl_sync(0xffffffffu, sz, owner);
                         const float y = __shfl_sync(0xffffffffu, gy, owner);
                         const float x = __shfl_sync(0xffffffffu, gx, owner);
-                        si[e] = super + (entry >> 5);
-                        float f0, f1;
-                        if constexpr (LEAN) {
-                            const float* m = xform_ptr(a.rot, si[e], 12);
-                            fz[e] = dot3(m[0], m[1], m[2], z, y, x);
-                            f0 = dot3(m[3], m[4], m[5], z, y, x);
-                            f1 = dot3(m[6], m[7], m[8], z, y, x);
-                        } else {
-                            fz[e] = grid2slice(z, y, x, a.scale, a.rot, si[e], a.ews, f0, f1);
+                        i = super + (entry >> 5);
+                        const float fz = locate(i, z, y, x, q0, q1);
+                        return at < n ? fz : 3.4e38f;
+                    };
+                    const auto keep = [&](int e, float2 v, float w1) {
+                        if (lane + 32 * e < n) {
+                            queue.value[lane + 32 * e] = v;
+                            queue.weight[lane + 32 * e] = w1;
                         }
-                        q0[e] = mul(f0, a.f_in0);
-                        q1[e] = mul(f1, a.f_in1);
-                    }
-                    float2 iv[2] = {};
-                    float iw[2] = {};
-                    if constexpr (LEAN && I == I_LINEAR) {
-                        using T = typename std::conditional<IN_C, float2, float>::type;
-                        const float2 window = window_of(pack2(fz[0], fz[1]));
+                    };
+                    if constexpr (InterpTraits<I>::SIZE <= 4) {
+                        // Both pairs' matrices and coordinates in flight together.
+                        int64_t si[2];
+                        float q0[2], q1[2], fz[2];
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            if (!(fabsf(fz[e]) < a.fb))
-                                continue;
-                            iw[e] = e ? window.y : window.x;
-                            const T* base = static_cast<const T*>(a.in.data) + si[e] * a.in.s0;
-                            if constexpr (IN_C)
-                                iv[e] = cmul(slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]), iw[e]);
-                            else
-                                iv[e].x = slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]) * iw[e];
-                            if (has_in_w) {
-                                const LinearCell cell(sp, q0[e], q1[e]);
-                                iw[e] = mul(cell.read(static_cast<const float*>(a.in_w.data) + si[e] * a.in_w.s0,
-                                                      static_cast<Idx>(a.in_w.s1), static_cast<Idx>(a.in_w.s2)).x, iw[e]);
+                        for (int e = 0; e < 2; ++e)
+                            fz[e] = prepare(e, si[e], q0[e], q1[e]);
+                        float2 iv[2] = {};
+                        float iw[2] = {};
+                        if constexpr (FORM == LEAN && I == I_LINEAR) {
+                            using T = typename std::conditional<IN_C, float2, float>::type;
+                            const float2 window = window_of(pack2(fz[0], fz[1]));
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                if (!(fabsf(fz[e]) < a.fb))
+                                    continue;
+                                iw[e] = e ? window.y : window.x;
+                                const T* base = static_cast<const T*>(a.in.data) + si[e] * a.in.s0;
+                                if constexpr (IN_C)
+                                    iv[e] = cmul(slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]), iw[e]);
+                                else
+                                    iv[e].x = slice_value(base, sp, static_cast<Idx>(a.in.s1), q0[e], q1[e]) * iw[e];
+                                if (has_in_w) {
+                                    const LinearCell cell(sp, q0[e], q1[e]);
+                                    iw[e] = mul(cell.read(static_cast<const float*>(a.in_w.data) + si[e] * a.in_w.s0,
+                                                          static_cast<Idx>(a.in_w.s1), static_cast<Idx>(a.in_w.s2)).x, iw[e]);
+                                }
+                            }
+                        } else {
+#pragma unroll 1
+                            for (int e = 0; 32 * e < n; ++e) {
+                                const float f = e ? fz[1] : fz[0];
+                                if (!(fabsf(f) < a.fb))
+                                    continue;
+                                float2 v;
+                                float w1;
+                                term(e ? si[1] : si[0], f, e ? q0[1] : q0[0], e ? q1[1] : q1[0], v, w1);
+                                (e ? iv[1] : iv[0]) = v;
+                                (e ? iw[1] : iw[0]) = w1;
                             }
                         }
+                        keep(0, iv[0], iw[0]);
+                        keep(1, iv[1], iw[1]);
                     } else {
+                        // The windows of 6 and 8 taps have no registers for a second pair (LANCZOS8 10 % slower).
 #pragma unroll 1
-                        for (int e = 0; e < 2; ++e) {
-                            const float f = e ? fz[1] : fz[0], c0 = e ? q0[1] : q0[0], c1 = e ? q1[1] : q1[0];
-                            const int64_t i = e ? si[1] : si[0];
-                            if (!(fabsf(f) < a.fb))
-                                continue;
-                            float w1 = windowed_sinc_fast(f, a.pfs, a.ifs, a.pfb);
-                            const float2 v1 = cmul(interp_spectrum_2d<I, IN_C>(a.in, sp, i, c0, c1), w1);
-                            if (has_in_w)
-                                w1 = mul(interp_spectrum_2d<I, false>(a.in_w, sp, i, c0, c1).x, w1);
-                            (e ? iv[1] : iv[0]) = v1;
-                            (e ? iw[1] : iw[0]) = w1;
-                        }
-                    }
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        if (lane + 32 * e < n) {
-                            queue.value[lane + 32 * e] = iv[e];
-                            queue.weight[lane + 32 * e] = iw[e];
+                        for (int e = 0; 32 * e < n; ++e) {
+                            int64_t i;
+                            float q0, q1, w1 = 0.f;
+                            float2 v = make_float2(0.f, 0.f);
+                            const float f = prepare(e, i, q0, q1);
+                            if (fabsf(f) < a.fb)
+                                term(i, f, q0, q1, v, w1);
+                            keep(e, v, w1);
                         }
                     }
                     __syncwarp();
@@ -307,15 +359,31 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                         const int k = g + lane;
                         const int listed = k < count ? list[k] : 0;
                         unsigned mask = k < count ? cut_mask : 0u;
-                        if (mask && cull)
-                            mask &= patch_mask(rotation_row0(a.rot, super + listed), patch, rows, first, 1.f / a.f_slice1,
+                        if (mask && cull && FORM == WALK)
+                            mask = patch_reaches(rotation_row0(a.rot, super + listed), patch, wbox, off, a.fb) ? mask : 0u;
+                        else if (mask && cull)
+                            mask &= patch_mask(rotation_row0(a.rot, super + listed), patch, rows, first, step,
                                                off, a.fb);
                         unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
                         while (todo) {
                             const int j = __ffs(todo) - 1;
                             todo &= todo - 1u;
                             const int index = __shfl_sync(0xffffffffu, listed, j);
-                            const unsigned pixels = __shfl_sync(0xffffffffu, mask, j);
+                            const unsigned pixels = FORM == WALK ? cut_mask : __shfl_sync(0xffffffffu, mask, j);
+                            if constexpr (FORM == WALK) {
+                                if (in_cut) {
+                                    float q0, q1;
+                                    const float fz = locate(super + index, sz, gy, gx, q0, q1);
+                                    if (fabsf(fz) < a.fb) {
+                                        float2 v;
+                                        float iw;
+                                        term(super + index, fz, q0, q1, v, iw);
+                                        value = cadd(value, v);
+                                        weight = add(weight, iw);
+                                    }
+                                }
+                                continue;
+                            }
                             if ((pixels >> lane) & 1u) {
                                 const int slot = (filled + __popc(pixels & ((1u << lane) - 1u))) & (2 * IE_HALF - 1);
                                 queue.entry[slot] = static_cast<unsigned>(index) << 5 | static_cast<unsigned>(lane);
@@ -331,7 +399,7 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
                         }
                     }
                 }
-                if (filled % IE_HALF)
+                if (FORM != WALK && filled % IE_HALF)
                     evaluate(filled / IE_HALF & 1, filled % IE_HALF);
                 __syncthreads();
             }
@@ -390,27 +458,53 @@ insert_extract_kernel(const __grid_constant__ ProjArgs a, int ntx, int tiles_per
     }
 }
 
+// The queue gathers the pixels that a slab covers only in part; it costs about 16 instructions per pair, and a
+// half that is not full runs with idle lanes. It therefore pays for thin slabs and for warps that meet many
+// pairs. `reach` is the slab's half-width in output pixels: within half a patch the lanes of WALK are mostly idle, from
+// 2 pixels on (1.5 for the windows of 6 and 8 taps, whose taps neighbouring lanes share in WALK) they are not. 700
+// slices of 64^2 to 8 of 64^2, us by WALK and by QUEUE (LINEAR by quaternions), half-widths of 1, 2, 3 and 6 pixels: 652 and
+// 406, 642 and 540, 640 and 640, 640 and 768; the LEAN form against WALK 645 and 354, 645 and 458, 640 and 525, 621 and 629.
+// A launch of many tiles that meet few slices each fills no halves: 64 slices to 48 of 256^2 take 88 us by WALK,
+// 90 by LEAN and 102 by QUEUE. With a curvature nothing is culled and most of the queue would be pairs outside the slabs.
+template<int I>
+Form form_of(const ProjArgs& a, int64_t n_tiles) {
+    const bool mat33 = a.rot.kind == 2 && a.scale.kind == 0, packed = I == I_LINEAR && mat33 && linear_slices(a);
+    const float reach = a.fb * a.f_slice1;
+    const float limit = packed ? 5.f : InterpTraits<I>::SIZE <= 4 ? 2.f : 1.5f;
+    const bool few = n_tiles > static_cast<int64_t>(sm_count()) * 8 ? a.n_in * 3 < a.slice_w : !packed && a.n_in < 8;
+    if (a.ews.on || reach > limit * 1.001f || few)
+        return WALK;
+    return packed || (I == I_NEAREST && mat33) ? LEAN : QUEUE;
+}
+
 template<int I, bool IN_C, bool OUT_C>
 cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
     const int wp = a.slice_w / 2 + 1;
     const int ntx = (wp + IE_TILE - 1) / IE_TILE, nty = (a.slice_h + IE_TILE - 1) / IE_TILE;
-    const int tiles_per_slice = ntx * nty;
-    const int64_t n_tiles = static_cast<int64_t>(tiles_per_slice) * a.n_slices;
+    const int64_t n_tiles = static_cast<int64_t>(ntx) * nty * a.n_slices;
     if (n_tiles == 0)
         return cudaSuccess;
     const int64_t max_grid = static_cast<int64_t>(sm_count()) * 8 * 16;
     const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    const bool lean = use_lean<I>(a);
-    if constexpr (I == I_LINEAR) {
-        if (lean && !a.in_slice_narrow) {
-            insert_extract_kernel<I, IN_C, OUT_C, true, int64_t><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
-            return cudaGetLastError();
-        }
+    // Fewer tiles are resident together in any order; those of one place next to each other, on the SMs of one
+    // TPC, are then slower (LANCZOS8, 16 slices to 8 of 128^2 with half-width 6: 219 us by slices, 269 us by places).
+    const bool by_place = n_tiles > static_cast<int64_t>(sm_count()) * 4;
+    switch (form_of<I>(a, n_tiles)) {
+        case LEAN:
+            if constexpr (I == I_LINEAR || I == I_NEAREST) {
+                if (I == I_NEAREST || a.in_slice_narrow)
+                    insert_extract_kernel<I, IN_C, OUT_C, LEAN, int><<<grid, IE_THREADS, 0, stream>>>(a, ntx, nty, n_tiles, by_place);
+                else if constexpr (I == I_LINEAR)
+                    insert_extract_kernel<I, IN_C, OUT_C, LEAN, int64_t><<<grid, IE_THREADS, 0, stream>>>(a, ntx, nty, n_tiles, by_place);
+            }
+            break;
+        case QUEUE:
+            insert_extract_kernel<I, IN_C, OUT_C, QUEUE><<<grid, IE_THREADS, 0, stream>>>(a, ntx, nty, n_tiles, by_place);
+            break;
+        case WALK:
+            insert_extract_kernel<I, IN_C, OUT_C, WALK><<<grid, IE_THREADS, 0, stream>>>(a, ntx, nty, n_tiles, by_place);
+            break;
     }
-    if (lean)
-        insert_extract_kernel<I, IN_C, OUT_C, true><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
-    else
-        insert_extract_kernel<I, IN_C, OUT_C, false><<<grid, IE_THREADS, 0, stream>>>(a, ntx, tiles_per_slice, n_tiles);
     return cudaGetLastError();
 }
 

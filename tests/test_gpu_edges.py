@@ -98,16 +98,42 @@ def test_linear_insertion_kernel(linear, kw):
     _check(default_case("insert", **{"seed": 707, **kw}), 1e-5)
 
 
-# The pair queue: fewer pairs than a half, halves that fill exactly and by many slices, a second pass of the
-# input slices (4096 each), the general rotation, windows over the whole slice, w offsets.
+# The pairs of insert_and_extract by the queue (LINEAR matrices two per lane, else one) and by walking: fewer
+# pairs than a half, halves that fill exactly and by many slices, a second pass of the input slices (4096
+# each), windows over the whole slice, w offsets, every value kind; slabs on either side of each form's
+# width (5, 2 and 1.5 pixels), and 8 and fewer slices.
 @pytest.mark.parametrize("kw", [dict(n=12, nslices=1, nout=2), dict(n=10, nslices=4200, nout=1, out_w=True),
                                 dict(n=33, nslices=64, nout=3, sinc=(0.03, 1.0), out_w=True, in_w=True),
+                                dict(n=33, nslices=64, nout=3, sinc=(0.03, 0.14), out_w=True, in_w=True),
                                 dict(n=20, nslices=40, nout=3, rot="quat", scale=True, sinc=(0.02, 0.2), out_w=True),
+                                dict(n=20, nslices=40, nout=3, rot="quat", scale=True, sinc=(0.02, 0.09), out_w=True),
+                                dict(n=10, nslices=4200, nout=1, rot="quat", out_w=True),
                                 dict(n=20, nslices=40, nout=2, sinc=(0.02, 0.1), w_sinc=(0.05, 0.2), out_w=True),
-                                dict(n=18, nslices=40, nout=2, in_dt="f32", out_dt="f32", interp="nearest")],
-                         ids=["few", "passes", "wide", "general", "w-window", "nearest"])
+                                dict(n=18, nslices=40, nout=2, in_dt="f32", out_dt="f32", interp="nearest"),
+                                dict(n=18, nslices=40, nout=2, in_dt="f32", out_dt="f32", interp="nearest", sinc=(0.06, 0.3))],
+                         ids=["few", "passes", "wide", "thick", "general", "general-thin", "general-passes", "w-window",
+                              "nearest", "nearest-wide"])
 def test_pair_queue(kw):
     _check(default_case("insert_extract", **{"remap": "h2h", "seed": 705, **kw}), 1e-5)
+
+
+@pytest.mark.parametrize("interp", ["cubic", "cubic_bspline", "lanczos4", "lanczos6", "lanczos8"])
+@pytest.mark.parametrize("kw", [dict(nslices=70, rot="quat"), dict(nslices=8, in_w=True), dict(nslices=7),
+                                dict(nslices=40, sinc=(0.05, 0.3), in_w=True), dict(nslices=40, in_dt="f32", out_dt="f32"),
+                                dict(nslices=40, w_sinc=(0.05, 0.12), out_dt="f32")],
+                         ids=["quat", "eight", "seven", "wide", "real", "w-window"])
+def test_pair_queue_windows(interp, kw):
+    _check(default_case("insert_extract", n=22, nout=3, remap="h2h", out_w=True, seed=708, interp=interp, **kw), 1e-5)
+
+
+# More tiles than are taken slice by slice (592): by place, rows alternately below and above the origin's, odd
+# and even numbers of rows, both layouts; and launches of many tiles that meet few slices each.
+@pytest.mark.parametrize("remap", ["h2h", "h2hc"])
+@pytest.mark.parametrize("kw", [dict(n=33, nout=110, nslices=30), dict(n=49, nout=80, nslices=200, rot="quat"),
+                                dict(n=64, nout=110, nslices=20), dict(n=64, nout=110, nslices=22, interp="nearest")],
+                         ids=["odd", "even", "few", "enough"])
+def test_tile_order(kw, remap):
+    _check(default_case("insert_extract", **{"remap": remap, "out_w": True, "seed": 711, **kw}), 1e-5)
 
 
 # LINEAR extraction: several slices per CTA with a shorter last group, rows past the slice, cells at the

@@ -67,6 +67,11 @@ __device__ __forceinline__ bool patch_reaches(const float3 n, const Patch& p, co
     return fabsf(centre) <= fb + half + 1e-5f * (1.f + fabsf(centre) + half);
 }
 
+// Columns lo to hi (0 <= lo <= 8, -1 <= hi <= 7) of a row of 8 pixels; none if hi < lo.
+__host__ __device__ constexpr unsigned row_columns(int lo, int hi) { return hi < lo ? 0u : (2u << hi) - (1u << lo); }
+static_assert(row_columns(0, 7) == 0xffu && row_columns(3, 5) == 0x38u && row_columns(7, 7) == 0x80u, "");
+static_assert(row_columns(0, -1) == 0u && row_columns(8, 7) == 0u && row_columns(8, -1) == 0u, "no shift is out of range");
+
 // The pixels of a warp's 4 x 8 patch (bit 8 row + column) that slice n may reach, fz being linear along a row.
 // `rows`: the rows' 2-D frequencies; `first`, `step`: the first column's frequency and the columns' spacing.
 __device__ __forceinline__ unsigned patch_mask(const float3 n, const Patch& p, const float (&rows)[4], float first,
@@ -84,7 +89,7 @@ __device__ __forceinline__ unsigned patch_mask(const float3 n, const Patch& p, c
         // Clamped before the conversions (NaN included: then the whole row, and the exact test decides).
         const int lo = __float2int_ru(fminf(fmaxf(fminf(a, b) - 1e-3f, 0.f), 8.f));
         const int hi = __float2int_rd(fmaxf(fminf(fmaxf(a, b) + 1e-3f, 7.f), -1.f));
-        mask |= ((2u << hi) - (1u << lo) & (hi >= lo ? 0xffu : 0u)) << 8 * r;
+        mask |= row_columns(lo, hi) << 8 * r;
     }
     return mask;
 }

@@ -80,7 +80,7 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
             for (int k = 0; k < SIZE; ++k)
                 w12[k] = pack2(w1[k], w1[k]);
         }
-        if (CPLX && __all_sync(0xffffffffu, cell.w != 0.f)) {
+        if (__all_sync(0xffffffffu, cell.w != 0.f)) {
             // Simple cells: one offset per pixel, rows and planes at the volume's strides from it. With 32-bit
             // byte offsets from the volume's base (Idx = uint32_t) a row costs one addition.
             const T* from = static_cast<const T*>(v.data);
@@ -91,21 +91,33 @@ __device__ __forceinline__ void window_samples(const View3<Idx>& v, const Spectr
             const Idx to_plane = v.s0 * static_cast<Idx>(sizeof(T)), to_row = v.s1 * static_cast<Idx>(sizeof(T));
 #pragma unroll 1
             for (int k0 = 0; k0 < SIZE; ++k0) {
-                unsigned long long e[SIZE], az = 0;
+                using E = typename std::conditional<CPLX, unsigned long long, float>::type;  // an element's bits
+                E e[SIZE];
                 Idx row = plane;
 #pragma unroll
                 for (int k = 0; k < SIZE; ++k) {
-                    e[k] = __ldg(reinterpret_cast<const unsigned long long*>(reinterpret_cast<const char*>(from) + row));
+                    e[k] = __ldg(reinterpret_cast<const E*>(reinterpret_cast<const char*>(from) + row));
                     row += to_row;
                 }
                 const float w0 = slot[4 + k0];
+                if constexpr (CPLX) {
+                    unsigned long long az = 0;
 #pragma unroll
-                for (int k = 0; k < SIZE; ++k)
-                    az = fma2(e[k], w12[k], az);
-                sum2 = fma2(az, pack2(w0, w0), sum2);
+                    for (int k = 0; k < SIZE; ++k)
+                        az = fma2(e[k], w12[k], az);
+                    sum2 = fma2(az, pack2(w0, w0), sum2);
+                } else {
+                    float az = 0.f;
+#pragma unroll
+                    for (int k = 0; k < SIZE; ++k)
+                        az = fmaf(e[k], w1[k], az);
+                    sum.x = fmaf(az, w0, sum.x);
+                }
                 plane += to_plane;
             }
-            sum = j < SIZE ? cmul(unpack2(sum2), slot[4 + 2 * S::AXIS + j]) : make_float2(0.f, 0.f);
+            if constexpr (CPLX)
+                sum = unpack2(sum2);
+            sum = j < SIZE ? cmul(sum, slot[4 + 2 * S::AXIS + j]) : make_float2(0.f, 0.f);
             group_sum<S, CPLX>(s, sum, j, at, n);
             continue;
         }

@@ -21,7 +21,7 @@ struct SpecArgs {
     float cz, cy, cx;          // phase centers (n / 2), as fractions of the sizes: c / n
 };
 
-// A block takes up to 256 columns of SPEC_ROWS consecutive rows (z, y) per thread row; a row's offsets and
+// A block takes up to 256 columns of up to SPEC_ROWS consecutive rows (z, y) per thread row; a row's offsets and
 // the z and y part of its phase are computed once, by one thread, and shared. One linear index per voxel,
 // taken apart by 64-bit divisions, cost more than the arithmetic: 250^3, 65 us ->
 // 45 us, against 24 us for its 156 MB.
@@ -29,11 +29,11 @@ constexpr int SPEC_ROWS = 4;
 constexpr int SPEC_MAX_ROWS = SPEC_ROWS * 8;  // of a block: at most 256 / 32 thread rows
 
 // Block: blockDim.x columns by blockDim.y thread rows; thread row y takes rows y, y + blockDim.y, ...
-__global__ void __launch_bounds__(256) spectrum_kernel(const __grid_constant__ SpecArgs a) {
+__global__ void __launch_bounds__(256) spectrum_kernel(const __grid_constant__ SpecArgs a, int rows_each) {
     __shared__ float s_turns[SPEC_MAX_ROWS];
     __shared__ int64_t s_value[SPEC_MAX_ROWS], s_weight[SPEC_MAX_ROWS];
     const int64_t rows = static_cast<int64_t>(a.d) * a.h;
-    const int per_block = static_cast<int>(blockDim.y) * SPEC_ROWS;
+    const int per_block = static_cast<int>(blockDim.y) * rows_each;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     for (int64_t first = blockIdx.y * static_cast<int64_t>(per_block); first < rows;
@@ -104,9 +104,14 @@ cudaError_t launch_reconstruction_spectrum(const nb_array* values, const nb_arra
             bx /= 2;
         const dim3 block(static_cast<unsigned>(bx), static_cast<unsigned>(256 / bx));
         const int64_t rows = static_cast<int64_t>(a.d) * a.h;
-        const int64_t groups = (rows + static_cast<int64_t>(block.y) * SPEC_ROWS - 1) / (static_cast<int64_t>(block.y) * SPEC_ROWS);
-        const dim3 grid(static_cast<unsigned>((a.wp + bx - 1) / bx), static_cast<unsigned>(groups < 65535 ? groups : 65535));
-        spectrum_kernel<<<grid, block, 0, stream>>>(a);
+        // Fewer rows per thread row where the launch would not give every SM its eight blocks.
+        const int64_t cols = (a.wp + bx - 1) / bx;
+        int rows_each = SPEC_ROWS;
+        while (rows_each > 1 && (rows + block.y * rows_each - 1) / (block.y * rows_each) * cols < sm_count() * 8)
+            rows_each /= 2;
+        const int64_t groups = (rows + static_cast<int64_t>(block.y) * rows_each - 1) / (static_cast<int64_t>(block.y) * rows_each);
+        const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(groups < 65535 ? groups : 65535));
+        spectrum_kernel<<<grid, block, 0, stream>>>(a, rows_each);
     }
     return cudaGetLastError();
 }

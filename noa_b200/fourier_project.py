@@ -257,11 +257,11 @@ def _options(interp="linear", fftfreq_cutoff=0.5, target_shape=None, ews_radius=
 def _stream_ptr(stream) -> int | None:
     torch = _torch()
     if stream is None:
-        # current_stream() without making its object, by private functions that another torch may not have
-        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-        device = getattr(torch._C, "_cuda_getDevice", None)
-        if raw and device and torch.cuda.is_initialized():
-            return raw(device())
+        if torch.cuda.is_initialized():
+            try:  # current_stream() without making its object, by private functions that another torch may not have
+                return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+            except AttributeError:
+                pass
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream

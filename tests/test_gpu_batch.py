@@ -196,7 +196,8 @@ def test_linear_batch_pair_copies_follow_volume_updates(tmp_path, monkeypatch):
     import torch
     from noa_b200.batch import ExtractBatch
     monkeypatch.setenv("NB_AUTOTUNE_CACHE", str(tmp_path / "autotune.txt"))
-    reqs, vols = _large_requests([(64, 300), (96, 150), (64, 40)], seed=9)
+    reqs, vols = _large_requests([(64, 1000), (96, 460), (64, 40)], seed=9)
+    assert _copies(reqs) == 2
     batch = ExtractBatch("hc2h", reqs, interp="linear", autotune=True)
     batch.run()
     torch.cuda.synchronize()
@@ -235,12 +236,13 @@ def test_linear_batch_scaled_and_curved_match_per_call(tmp_path, monkeypatch):
     from noa_b200 import synthetic
     from noa_b200.batch import ExtractBatch
     monkeypatch.setenv("NB_AUTOTUNE_CACHE", str(tmp_path / "autotune.txt"))
-    reqs, _ = _large_requests([(64, 300), (48, 400)], seed=13)
+    reqs, _ = _large_requests([(64, 1000), (48, 1800)], seed=13)
     for i, r in enumerate(reqs):
         count = r.slice_shape[0]
         sc = synthetic.scale_matrices(count, (1.0, 1.0), seed=80 + i, jitter=0.05).astype(np.float32)
         r.inv_scaling = torch.from_numpy(sc).cuda()
     ews = (45.0, 60.0)
+    assert _copies(reqs, ews_radius=ews) == 2
     batch = ExtractBatch("hc2h", reqs, interp="linear", ews_radius=ews, autotune=False)
     batch.run()
     torch.cuda.synchronize()

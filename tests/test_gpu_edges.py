@@ -58,13 +58,17 @@ def test_rasterize_run_lengths(nslices):
 
 
 # The planes that a pixel's z samples share: more samples than planes of the volume, offsets outside it, a
-# window wider than the table, odd sizes, power spectra.
-@pytest.mark.parametrize("kw", [dict(n=16, w_sinc=(0.05, 0.9), cutoff=0.9), dict(n=17, w_sinc=(-1.0, 0.2), remap="h2h"),
-                                dict(n=64, nslices=160, w_sinc=(0.1, 0.6), cutoff=0.7),
-                                dict(n=20, w_sinc=(-1.0, 0.15), out_dt="f32")],
-                         ids=["beyond", "odd", "long", "power"])
-def test_w_window_planes(kw):
-    _check(default_case("extract", **{"nslices": 48, "remap": "hc2h", "out_w": True, "seed": 703, **kw}), 1e-5)
+# window wider than the table, odd sizes, power spectra; from a pair copy and from the volume.
+@pytest.mark.parametrize("copies", [0, 1])
+@pytest.mark.parametrize("kw", [dict(n=16, w_sinc=(0.05, 0.9), cutoff=0.9, nslices=520), dict(n=64, w_sinc=(0.1, 0.6), cutoff=0.7, nslices=160),
+                                dict(n=17, w_sinc=(-1.0, 0.2), remap="h2h", nslices=2000),
+                                dict(n=20, w_sinc=(-1.0, 0.15), out_dt="f32", nslices=2000)],
+                         ids=["beyond", "long", "odd", "power"])
+def test_w_window_planes(kw, copies):
+    case = default_case("extract", **{"remap": "hc2h", "out_w": True, "seed": 703, **kw})
+    if not copies:
+        case["nslices"] = 8
+    _check(case, 1e-5, copies)
 
 
 # LINEAR insertion from Mat33 rotations: bricks that the volume fills partly, more slices than one pass of
@@ -157,27 +161,53 @@ def test_linear_extraction_groups(kw, copies, remap):
     _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5, copies)
 
 
-# The rule on making a pair copy (three pixels per voxel, 2 M pixels), its padded strides, and requests of a
-# batch that read their volume in grids of their own: the same bits with and without the copy.
-@pytest.mark.parametrize("n,size,count", [(33, 33, 4000), (64, 64, 1100), (96, 95, 470), (40, 200, 110), (128, 128, 250)])
-def test_extraction_with_and_without_pair_copy(n, size, count):
+# The rule on making a pair copy (two pixels per voxel, 3 * 2^19 pixels), its padded strides, and requests of a
+# batch that read their volume in grids of their own: the same bits with and without the copy, in every layout
+# and with every form of the coordinates and outputs that a copy serves.
+def _with_and_without_pair_copy(n, size, count, remap="hc2h", form="plain"):
+    import gpu_run
     import torch
     from noa_b200 import fourier_project as fp, synthetic
     from noa_b200.batch import ExtractBatch, ExtractRequest
-    vol = torch.from_numpy(synthetic.make_volume(n, seed=n)).cuda()
-    rot = fp.pack_rotations(torch.from_numpy(synthetic.random_rotations(count, seed=count)).cuda())
+    q = synthetic.random_quaternions(count, seed=count)
+    rot = torch.from_numpy(q.astype(np.float32)).cuda() if form == "quaternion" else \
+        fp.pack_rotations(torch.from_numpy(synthetic.quaternion_to_matrix(q).astype(np.float32)).cuda())
+    vol = synthetic.make_volume(n, seed=n)  # centered
+    if remap.startswith("h2"):
+        vol = np.ascontiguousarray(np.fft.ifftshift(vol, axes=(1, 2)))
+    vol = torch.from_numpy(vol).cuda()
+    scale = torch.from_numpy(synthetic.scale_matrices(count, (1.0, 1.0), seed=5, jitter=0.05).astype(np.float32)).cuda() \
+        if form == "scaled" else None
+    kw = {"curved": dict(ews_radius=(45.0, 60.0)), "cutoff": dict(fftfreq_cutoff=0.8)}.get(form, {})
     shape, slices = (1, n, n, n), (count, 1, size, size)
-    outs = [torch.empty((count, 1, size, size // 2 + 1), dtype=torch.complex64, device="cuda") for _ in range(3)]
-    try:
-        for out, limit in zip(outs, (None, 0)):
-            fp.set_scratch_limit(limit)
-            fp.extract_central_slices_3d("hc2h", vol, None, shape, out, None, slices, None, rot)
-    finally:
-        fp.set_scratch_limit(None)
-    batch = ExtractBatch("hc2h", [ExtractRequest(volume=vol, volume_shape=shape, slice=outs[2], slice_shape=slices,
-                                                 fwd_rotation=rot)], autotune=False)
+    dt = torch.float32 if form == "power" else torch.complex64
+    outs = [torch.empty((count, 1, size, size // 2 + 1), dtype=dt, device="cuda") for _ in range(3)]
+    weights = [torch.empty(outs[0].shape, device="cuda") if form == "weights" else None for _ in range(3)]
+
+    def extract(k):
+        fp.extract_central_slices_3d(remap, vol, None, shape, outs[k], weights[k], slices, scale, rot, **kw)
+    extract(0)
+    assert gpu_run.scratch_wanted(lambda: extract(1))[0] == 1
+    batch = ExtractBatch(remap, [ExtractRequest(volume=vol, volume_shape=shape, slice=outs[2], slice_shape=slices,
+                                                slice_weight=weights[2], inv_scaling=scale, fwd_rotation=rot)],
+                         autotune=False, **kw)
     batch.run()
     torch.cuda.synchronize()
     assert batch.info()["n_direct"] == 1
+    assert outs[0].abs().max().item() > 0
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    if form == "weights":
+        assert torch.equal(weights[0], weights[1]) and torch.equal(weights[0], weights[2])
     batch.close()
+
+
+@pytest.mark.parametrize("n,size,count", [(33, 33, 4000), (64, 64, 1100), (96, 95, 470), (40, 200, 110), (128, 128, 400)])
+def test_extraction_with_and_without_pair_copy(n, size, count):
+    _with_and_without_pair_copy(n, size, count)
+
+
+@pytest.mark.parametrize("remap", ["h2h", "h2hc", "hc2h", "hc2hc"])
+@pytest.mark.parametrize("form", ["plain", "power", "weights", "quaternion", "scaled", "curved", "cutoff"])
+def test_forms_with_and_without_pair_copy(form, remap):
+    _with_and_without_pair_copy(33, 33, 4000, remap, form)
+    _with_and_without_pair_copy(40, 51, 1600, remap, form)

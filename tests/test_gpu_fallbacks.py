@@ -54,11 +54,14 @@ def test_limit_is_reported_and_removed(cap):
 @pytest.mark.parametrize("remap", ["hc2h", "h2hc"])
 def test_extract_without_pair_copy(cap, remap):
     import gpu_run
-    call = build(default_case("extract", n=64, nslices=64, remap=remap, seed=701))  # pair path when uncapped
+    from noa_b200 import fourier_project as fp
+    call = build(default_case("extract", n=64, nslices=1000, remap=remap, seed=701))  # pair path when uncapped
     ref = _oracle(call)
     fast, _ = gpu_run.run(clone(call))
     cap(0)
+    before = fp.scratch_refusals()
     slow, _ = gpu_run.run(clone(call))
+    assert fp.scratch_refusals() == before + 1
     assert rel_l2(slow, ref.out) <= 1e-5
     np.testing.assert_array_equal(slow, fast)
 
@@ -103,7 +106,7 @@ def _batch_requests():
     from noa_b200 import synthetic
     from noa_b200.batch import ExtractRequest
     reqs, specs = [], []
-    for i, (n, count) in enumerate([(64, 300), (48, 9)]):
+    for i, (n, count) in enumerate([(64, 1000), (48, 9)]):
         vol = torch.from_numpy(synthetic.make_volume(n, seed=710 + i)).cuda()
         rot = torch.from_numpy(synthetic.random_rotations(count, seed=720 + i)).cuda()
         out = torch.zeros((count, 1, n, n // 2 + 1), dtype=torch.complex64, device="cuda")
@@ -133,7 +136,9 @@ def test_batch_without_pair_copies_matches_per_call(cap):
     from noa_b200 import fourier_project as fp
     reqs, specs = _batch_requests()
     cap(1 << 20)
+    before = fp.scratch_refusals()
     b = batch.ExtractBatch("hc2h", reqs, autotune=False)
+    assert fp.scratch_refusals() == before + 1
     b.run()
     torch.cuda.synchronize()
     cap(None)

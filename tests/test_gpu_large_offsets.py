@@ -33,9 +33,10 @@ def big_buffer():
     torch.cuda.empty_cache()
 
 
-@pytest.mark.parametrize("count", [8, 400], ids=["generic", "pair_copy"])
+@pytest.mark.parametrize("count", [8, 1000], ids=["generic", "pair_copy"])
 def test_extract_from_a_volume_spanning_2_31_elements(big_buffer, count):
     import torch
+    import gpu_run
     from noa_b200 import fourier_project as fp
     from noa_b200 import synthetic
     compact = torch.from_numpy(synthetic.make_volume(N, seed=31)).cuda()
@@ -46,7 +47,12 @@ def test_extract_from_a_volume_spanning_2_31_elements(big_buffer, count):
     outs = []
     for vol in (wide, compact):
         o = torch.full((count, 1, N, N // 2 + 1), 7, dtype=torch.complex64, device="cuda")
-        fp.extract_central_slices_3d("hc2h", vol, None, (1, N, N, N), o, None, (count, 1, N, N), None, rot)
+
+        def extract():
+            fp.extract_central_slices_3d("hc2h", vol, None, (1, N, N, N), o, None, (count, 1, N, N), None, rot)
+        assert gpu_run.scratch_wanted(extract)[0] == (count == 1000)
+        o.fill_(7)
+        extract()
         outs.append(o)
     torch.cuda.synchronize()
     assert outs[1].abs().max().item() > 0
@@ -115,3 +121,36 @@ def test_insertions_from_slices_spanning_2_31_elements(big_buffer):
     for a, b in ((gs, gs2), (gr, gr2)):  # atomic scatters: summation order only
         rel = float(((a - b).abs().pow(2).sum() / b.abs().pow(2).sum()).sqrt())
         assert rel <= 1e-6, rel
+
+
+# The window extraction's offsets: 32-bit byte offsets from the volume's start (signed they would be negative
+# from 2 GiB on), and 64-bit ones past 4 GiB; as a call and in a batch (which takes volumes of fewer than
+# 2^31 elements).
+@pytest.mark.parametrize("interp", ["cubic", "lanczos8"])
+@pytest.mark.parametrize("real", [False, True], ids=["complex", "real"])
+@pytest.mark.parametrize("gib", [3, 6, 12])
+def test_window_extraction_offsets(big_buffer, interp, real, gib):
+    import torch
+    from noa_b200 import fourier_project as fp
+    from noa_b200 import synthetic
+    from noa_b200.batch import ExtractBatch, ExtractRequest
+    wp, count = N // 2 + 1, 6
+    buf = big_buffer.view(torch.float32) if real else big_buffer
+    compact = torch.from_numpy(synthetic.make_volume(N, seed=41)).cuda()
+    if real:
+        compact = compact.real.contiguous()
+    depth = gib * 2 ** 30 // compact.element_size() // (N - 1)
+    wide = torch.as_strided(buf, (1, N, N, wp), (N * depth, depth, wp, 1))
+    wide.copy_(compact)
+    rot = fp.pack_rotations(torch.from_numpy(synthetic.random_rotations(count, seed=42)).cuda())
+    sshape, dt = (count, 1, N, N), torch.float32 if real else torch.complex64
+    outs = [torch.full((count, 1, N, wp), 7, dtype=dt, device="cuda") for _ in range(3)]
+    for vol, o in ((wide, outs[0]), (compact, outs[1])):
+        fp.extract_central_slices_3d("hc2h", vol, None, (1, N, N, N), o, None, sshape, None, rot, interp=interp)
+    assert outs[1].abs().max().item() > 0 and torch.equal(outs[0], outs[1])
+    if (N - 1) * depth < 2 ** 31 - 2 ** 20:
+        batch = ExtractBatch("hc2h", [ExtractRequest(volume=wide, volume_shape=(1, N, N, N), slice=outs[2],
+                                                     slice_shape=sshape, fwd_rotation=rot)], interp=interp, autotune=False)
+        batch.run()
+        assert torch.equal(outs[2], outs[1])
+        batch.close()

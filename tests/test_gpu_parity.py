@@ -141,14 +141,21 @@ def test_gpu_constant_input_rasterize():
 @pytest.mark.parametrize("remap", ["h2h", "h2hc", "hc2h", "hc2hc"])
 @pytest.mark.parametrize("out_dt", ["c32", "f32"])
 def test_gpu_extract_pair_path(remap, out_dt):
-    """Enough slices that extraction takes the pair-copy fast path (pixels >= 2 x voxels)."""
+    """Enough slices that extraction takes the pair-copy fast path (at least 3 * 2^19 pixels, 2 per voxel)."""
     import gpu_run
-    call = build(default_case("extract", remap=remap, n=32, nslices=80, out_dt=out_dt, out_w=True, seed=640))
+    call = build(default_case("extract", remap=remap, n=32, nslices=3900, out_dt=out_dt, out_w=True, seed=640))
     ref = clone(call)
     FpOracle().run(ref, 8)
+    assert _copies(call) == 1
     out, out_w = gpu_run.run(clone(call))
     assert rel_l2(out, ref.out) <= 1e-5
     assert rel_l2(out_w, ref.out_w) <= 1e-5
+
+
+def _copies(call):
+    """How many pair copies the library makes for the call."""
+    import gpu_run
+    return gpu_run.scratch_wanted(lambda: gpu_run.run(clone(call)))[0]
 
 
 def _generic_forced(call):
@@ -165,7 +172,8 @@ def test_gpu_extract_pair_path_bit_identical_to_generic(variant):
     curvature (which the pair kernels compute through the same slice2grid)."""
     import gpu_run
     kw = {"scaled": dict(scale=True), "ews": dict(ews=(45.0, 60.0))}.get(variant, {})
-    call = build(default_case("extract", remap="hc2h", n=48, nslices=96, seed=641, **kw))
+    call = build(default_case("extract", remap="hc2h", n=48, nslices=1800, seed=641, **kw))
+    assert _copies(call) == 1 and _copies(_generic_forced(call)) == 0
     a, _ = gpu_run.run(clone(call))
     b, _ = gpu_run.run(_generic_forced(call))
     np.testing.assert_array_equal(a, b)
@@ -176,9 +184,10 @@ def test_gpu_extract_pair_path_scaled_or_curved(variant):
     """Scaled and curved extractions through the pair copy, against the oracle."""
     import gpu_run
     kw = {"scaled": dict(scale=True), "ews": dict(ews=(45.0, 60.0))}[variant]
-    call = build(default_case("extract", remap="h2hc", n=32, nslices=80, out_w=True, seed=644, **kw))
+    call = build(default_case("extract", remap="h2hc", n=32, nslices=3900, out_w=True, seed=644, **kw))
     ref = clone(call)
     FpOracle().run(ref, 8)
+    assert _copies(call) == 1
     out, out_w = gpu_run.run(clone(call))
     assert rel_l2(out, ref.out) <= 1e-5
     assert rel_l2(out_w, ref.out_w) <= 1e-5
@@ -187,12 +196,13 @@ def test_gpu_extract_pair_path_scaled_or_curved(variant):
 @pytest.mark.parametrize("remap", ["h2h", "hc2hc"])
 @pytest.mark.parametrize("out_dt", ["c32", "f32"])
 def test_gpu_extract_pair_path_w_window(remap, out_dt):
-    """The w-windowed extraction through the pair copy (5-sample window, enough slices)."""
+    """The w-windowed extraction through the pair copy (5-sample window, at least 2^21 samples)."""
     import gpu_run
-    call = build(default_case("extract", remap=remap, n=32, nslices=80, out_dt=out_dt, out_w=True,
+    call = build(default_case("extract", remap=remap, n=32, nslices=800, out_dt=out_dt, out_w=True,
                               w_sinc=(1.5 / 32, 3.0 / 32), seed=642))
     ref = clone(call)
     FpOracle().run(ref, 8)
+    assert _copies(call) == 1
     out, out_w = gpu_run.run(clone(call))
     assert rel_l2(out, ref.out) <= 1e-5
     assert rel_l2(out_w, ref.out_w) <= 1e-5
@@ -201,8 +211,9 @@ def test_gpu_extract_pair_path_w_window(remap, out_dt):
 def test_gpu_extract_pair_path_w_window_bit_identical_to_generic():
     """With the w-window too, the pair path and the generic path give identical bits."""
     import gpu_run
-    call = build(default_case("extract", remap="hc2h", n=48, nslices=96, out_w=True, w_sinc=(2.0 / 48, 4.0 / 48),
+    call = build(default_case("extract", remap="hc2h", n=48, nslices=300, out_w=True, w_sinc=(2.0 / 48, 4.0 / 48),
                               seed=643))
+    assert _copies(call) == 1 and _copies(_generic_forced(call)) == 0
     a, _ = gpu_run.run(clone(call))
     b, _ = gpu_run.run(_generic_forced(call))
     np.testing.assert_array_equal(a, b)

@@ -1,7 +1,7 @@
 // Batched extraction: many extract_central_slices_3d calls — different volumes, box sizes and slice
-// counts — executed by ONE persistent kernel, replayed as a CUDA graph; LINEAR requests read through
-// pair copies with enough pixels run instead as grids of the per-call pair kernel on parallel graph
-// branches (nb_extract_batch_t::direct).
+// counts — executed by ONE persistent kernel, replayed as a CUDA graph; LINEAR requests with enough
+// pixels run instead as grids of the per-call kernels on parallel graph branches
+// (nb_extract_batch_t::direct).
 //
 // Work decomposition: every request is cut into (slice, tile) items, a tile being TY x TX pixels of
 // one output slice (4 TY x TX for a request read through its volume's pair copy, 4 rows per thread).
@@ -66,7 +66,7 @@ constexpr int N_SIDE = 4;  // graph branches the direct grids alternate on
 constexpr int64_t ONESHOT_DIRECT_MIN_PIXELS = int64_t(1) << 21;
 
 // PAIRS_PPT output pixels (rows y0, y0 + dy, ...) of column u read through the volume's pair copy:
-// the body of extract_pairs_kernel (fp_extract.cu).
+// the body of extract_linear_kernel (fp_extract.cu).
 template<bool OUT_C>
 __device__ __forceinline__ void extract_rows_pairs(const ProjArgs& a, const float4* pairs, int64_t b, int y0,
                                                    int dy, int u) {

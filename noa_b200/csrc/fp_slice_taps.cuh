@@ -28,13 +28,14 @@ struct WindowPair {
         const auto both = [](float v) { return pack2(v, v); };
         z &= 0x7fffffff7fffffffull;
         const unsigned long long xs = fma2(z, pfs, both(PI_TINY)), s = fma2(z, ifs, both(TINY));
-        const unsigned long long t = add2(s, both(12582912.f));  // rounds to integers, as sinpi_reduced
-        const unsigned long long r = fma2(add2(t, both(-12582912.f)), both(-1.f), s);
+        const unsigned long long t = add2(s, both(SINPI_ROUND));  // rounds to integers, as sinpi_reduced
+        const unsigned long long r = fma2(add2(t, both(-SINPI_ROUND)), both(-1.f), s);
         const unsigned long long u = mul2(r, r);
-        unsigned long long p = fma2(both(0.07756046f), u, both(-0.59824216f));
-        p = fma2(p, u, both(2.5500698f));
-        p = fma2(p, u, both(-5.16771f));
-        p = fma2(p, u, both(3.1415927f));
+        constexpr float C[5] = NB_SINPI;
+        unsigned long long p = fma2(both(C[0]), u, both(C[1]));
+#pragma unroll
+        for (int k = 2; k < 5; ++k)
+            p = fma2(p, u, both(C[k]));
         const float2 x = unpack2(xs), b = unpack2(mul2(z, pfb));
         float2 sn = unpack2(mul2(r, p)), inv;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(x.x));

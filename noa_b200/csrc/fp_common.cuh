@@ -197,7 +197,7 @@ __device__ __forceinline__ float windowed_sinc(float fftfreq, float fftfreq_sinc
 }
 
 // sin(pi |s|), for |s| < 2^22: |s| minus the nearest integer (exact), an odd polynomial on [-1/2, 1/2] and
-// the sign of the integer's parity. The polynomial's five terms (SINPI, highest first) are a fit for the smallest
+// the sign of the integer's parity. The polynomial's five terms (NB_SINPI, highest first) are a fit for the smallest
 // relative error, 5.3e-9 before its coefficients are rounded to single precision; the result is within 1.7e-7 (2.8
 // ulp) of the sine, 5e-8 in the mean square (emulated over phases up to 2^20).
 #define NB_SINPI {0.07756046f, -0.59824216f, 2.5500698f, -5.16771f, 3.1415927f}
@@ -386,6 +386,13 @@ struct SliceReader {
     }
 };
 
+// A floored coordinate as the index of its cell. Huge and infinite ones (an infinite matrix element, a scaling of
+// 1e12) stop short of the ends of the integers, so that the taps' offsets from the cell do not wrap
+// around into the spectrum; they meet no tap either way. NaN gives 0, and NaN weights.
+__device__ __forceinline__ int cell_index(float floored) {
+    return min(max(static_cast<int>(floored), -(1 << 30)), 1 << 30);
+}
+
 // interpolate_spectrum, 2-D (slice) form; `batch` selects the slice.
 template<int I, bool CPLX>
 __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const Spectrum2& sp, int64_t batch,
@@ -410,7 +417,7 @@ __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const S
     } else {
         constexpr int START = -(SIZE - 1) / 2;
         const float fl0 = floorf(f0), fl1 = floorf(f1);
-        const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1);
+        const int b0 = cell_index(fl0), b1 = cell_index(fl1);
         float w0[SIZE], w1[SIZE];
         interp_weights<I>(sub(f0, fl0), w0);
         interp_weights<I>(sub(f1, fl1), w1);

@@ -102,6 +102,39 @@ def test_linear_insertion_kernel(linear, kw):
     _check(default_case("insert", **{"seed": 707, **kw}), 1e-5)
 
 
+# In-slice coordinates past the range of the integers: no tap of the slice is read, as for coordinates that are
+# outside it by less. A slice scaled by 1e15 adds what one scaled by 1e7 adds; one whose in-plane matrix rows are
+# infinite leaves the voxels and pixels outside its slab as they are.
+@pytest.mark.parametrize("interp", ["nearest", "linear", "cubic", "cubic_bspline", "lanczos4", "lanczos6", "lanczos8"])
+@pytest.mark.parametrize("func", ["insert", "scatter", "insert_extract"])
+@pytest.mark.parametrize("kw", [dict(), dict(rot="quat"), dict(sinc=(0.05, 0.3)), dict(in_dt="f32", out_dt="f32", in_w=True, out_w=True)],
+                         ids=["thin", "quat", "thick", "real"])
+def test_coordinates_past_the_integers(interp, func, kw):
+    import gpu_run
+    call = build(default_case(func.replace("scatter", "insert"), interp=interp, n=24, nslices=12, remap="h2h", scale=True,
+                              seed=712, **kw))
+    scatter = func == "scatter"
+    outs = []
+    for factor in (1e7, 1e15):
+        c = clone(call)
+        c.scale = call.scale.copy()
+        c.scale[5] *= np.float32(factor)
+        outs.append(gpu_run.run(c, scatter=scatter)[0])
+    assert np.isfinite(outs[0]).all() and np.abs(outs[0]).max() > 0
+    assert rel_l2(outs[1], outs[0]) <= 1e-6 if scatter else np.array_equal(outs[0], outs[1])
+    if call.rot.shape[1:] == (3, 3) and interp != "nearest":  # which takes a voxel for NaN coordinates (inf * 0)
+        c = clone(call)
+        c.scale, c.rot = None, call.rot.copy()
+        base = clone(c)
+        base.rot[5, 1:] *= np.float32(1e7)
+        outs = [gpu_run.run(base, scatter=scatter)[0]]
+        c.rot = call.rot.copy()
+        c.rot[5, 1:] = np.inf
+        outs.append(gpu_run.run(c, scatter=scatter)[0])
+        same = np.isfinite(outs[1])
+        assert same.any() and rel_l2(outs[1][same], outs[0][same]) <= (1e-6 if scatter else 0)
+
+
 # The pairs of insert_and_extract by the queue (LINEAR matrices two per lane, else one) and by walking: fewer
 # pairs than a half, halves that fill exactly and by many slices, a second pass of the input slices (4096
 # each), windows over the whole slice, w offsets, every value kind; slabs on either side of each form's

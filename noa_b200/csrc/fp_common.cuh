@@ -386,13 +386,6 @@ struct SliceReader {
     }
 };
 
-// A floored coordinate as the index of its cell. Huge and infinite ones (an infinite matrix element, a scaling of
-// 1e12) stop short of the ends of the integers, so that the taps' offsets from the cell do not wrap
-// around into the spectrum; they meet no tap either way. NaN gives 0, and NaN weights.
-__device__ __forceinline__ int cell_index(float floored) {
-    return min(max(static_cast<int>(floored), -(1 << 30)), 1 << 30);
-}
-
 // interpolate_spectrum, 2-D (slice) form; `batch` selects the slice.
 template<int I, bool CPLX>
 __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const Spectrum2& sp, int64_t batch,
@@ -417,15 +410,17 @@ __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const S
     } else {
         constexpr int START = -(SIZE - 1) / 2;
         const float fl0 = floorf(f0), fl1 = floorf(f1);
-        const int b0 = cell_index(fl0), b1 = cell_index(fl1);
+        const int b0 = static_cast<int>(fl0), b1 = static_cast<int>(fl1);
         float w0[SIZE], w1[SIZE];
         interp_weights<I>(sub(f0, fl0), w0);
         interp_weights<I>(sub(f1, fl1), w1);
         float2 value = make_float2(0.f, 0.f);
         {
-            // Interior fast path (all taps in bounds, none flipped per tap): same terms, same order.
-            constexpr int END = SIZE / 2;
-            if (b0 + START >= lo0 && b0 + END <= hi0 && b1 + START >= 0 && b1 + END <= hi1) {
+            // Interior fast path (all taps in bounds, none flipped per tap): same terms, same order. Compared modulo 2^32, so
+            // that the cell of an infinite or huge coordinate, INT_MAX or INT_MIN, is outside whatever is added to it.
+            const unsigned rows = max(sp.n0 - SIZE + 1, 0), columns = max(hi1 - SIZE + 2, 0);  // of such cells
+            if (static_cast<unsigned>(b0) + static_cast<unsigned>(START - lo0) < rows &&
+                static_cast<unsigned>(b1) + static_cast<unsigned>(START) < columns) {
 #pragma unroll
                 for (int y = 0; y < SIZE; ++y) {
                     const int iy = frequency2index(sp.centered, b0 + START + y, sp.n0);
@@ -445,10 +440,13 @@ __device__ __forceinline__ float2 interp_spectrum_2d(const SrcView& src, const S
             float2 vy = make_float2(0.f, 0.f);
 #pragma unroll
             for (int x = 0; x < SIZE; ++x) {
-                int t0 = b0 + START + y, t1 = b1 + START + x;
+                // Modulo 2^32: a tap that wraps around is as far outside as its cell.
+                int t0 = static_cast<int>(static_cast<unsigned>(b0) + static_cast<unsigned>(START + y));
+                int t1 = static_cast<int>(static_cast<unsigned>(b1) + static_cast<unsigned>(START + x));
                 float conj = 1.f;
                 if (!FLIP_EARLY && t1 < 0) {
-                    t0 = -t0; t1 = -t1;
+                    t0 = static_cast<int>(0u - static_cast<unsigned>(t0));
+                    t1 = static_cast<int>(0u - static_cast<unsigned>(t1));
                     conj = -1.f;
                 }
                 if (t0 >= lo0 && t0 <= hi0 && t1 >= 0 && t1 <= hi1) {

@@ -213,9 +213,9 @@ __device__ __forceinline__ void extract_window_patch(const ProjArgs& a, int64_t 
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const float fl = floorf(q[k]);
-                // NaN (which the w-window's cutoff test lets pass) meets taps, whose weights carry it into the value,
-                // as in the other interpolations.
-                cell[k] = cell_index(fl);
+                // Far outside (infinities included): no tap either way. NaN (which the w-window's cutoff test lets pass) meets
+                // taps, whose weights carry it into the value, as in the other interpolations.
+                cell[k] = fl != fl ? 0 : static_cast<int>(fminf(fmaxf(fl, -1e9f), 1e9f));
                 interp_weights<I>(sub(q[k], fl), ws[k]);
             }
             float4* slot = reinterpret_cast<float4*>(s.slot[at]);

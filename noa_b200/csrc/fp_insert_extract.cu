@@ -110,10 +110,12 @@ enum Form {
 };
 
 // Resident CTAs per SM asked of the compiler. WALK: 5 (48 registers; with 6 3 % slower for quaternions and scaling,
-// equal for matrices). The wider windows: 2, where the compiler's choice for the queue was one, up to 1.4 times
-// slower.
+// equal for matrices), 2 for the wider windows. The queue's wider windows ask for none: they stay within the 128
+// registers of two, and with two asked for (104 registers) are 1.5 % slower on average, up to 7 %.
 template<int I, Form FORM>
-constexpr int insert_extract_min_ctas() { return I != I_LINEAR && I != I_NEAREST ? 2 : FORM == WALK ? 5 : 4; }
+constexpr int insert_extract_min_ctas() {
+    return FORM == WALK ? (I != I_LINEAR && I != I_NEAREST ? 2 : 5) : (I != I_LINEAR && I != I_NEAREST ? 1 : 4);
+}
 
 template<int I, bool IN_C, bool OUT_C, Form FORM, typename Idx = int>
 __global__ void __launch_bounds__(IE_THREADS, insert_extract_min_ctas<I, FORM>())

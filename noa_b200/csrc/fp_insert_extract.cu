@@ -493,9 +493,11 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
         return cudaSuccess;
     const int64_t max_grid = static_cast<int64_t>(sm_count()) * 8 * 16;
     const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    // Fewer tiles are resident together in any order; those of one place next to each other, on the SMs of one
-    // TPC, are then slower (LANCZOS8, 16 slices to 8 of 128^2 with half-width 6: 219 us by slices, 269 us by places).
-    const bool by_place = n_tiles > static_cast<int64_t>(sm_count()) * 4;
+    // Few tiles are resident together in any order; those of one place next to each other, on the SMs of one TPC,
+    // are then slower. By slices and by places: 64 slices to 8 of 128^2 (320 tiles), half-width 6, LANCZOS8 935 and 1006
+    // us, CUBIC 183 and 181; 700 to 48 of 64^2 (576 tiles) LANCZOS8 20.3 and 18.9 ms, CUBIC 3.10 and 2.58, LINEAR 0.70
+    // and 0.64.
+    const bool by_place = n_tiles > static_cast<int64_t>(sm_count()) * 3;
     switch (form_of<I>(a, n_tiles)) {
         case LEAN:
             if constexpr (I == I_LINEAR || I == I_NEAREST) {

@@ -56,8 +56,8 @@ enum { NB_BATCH_AUTOTUNE = 1, NB_BATCH_PERSISTENT_ONLY = 2 };
  * so it writes the outputs) and captures the launch into a CUDA graph. Synchronizes `stream`.
  * LINEAR batches over complex volumes (no input weights or w-window) hold a pair copy (16 bytes per
  * rfft voxel, rows and planes padded by a few elements) of each volume whose requests read at least two
- * output pixels per voxel of it (three of a volume of 2^24 voxels and more, for requests run as grids); the graph rebuilds these copies at every run, so
- * changes to the volumes between runs are seen. A LINEAR request with at least 2^16 output pixels runs,
+ * output pixels per voxel of it (three of a volume of 2^24 voxels and more, for requests run as grids); the
+ * graph rebuilds these copies at every run, so changes to the volumes between runs are seen. A LINEAR request with at least 2^16 output pixels runs,
  * in the graph, as a grid of its own (the per-call kernel) on a parallel branch, from its volume or, once
  * it is written, from its volume's copy; the copies are made meanwhile on a higher-priority branch
  * (NB_BATCH_PERSISTENT_ONLY keeps every request in the persistent kernel).
@@ -93,8 +93,8 @@ typedef struct {
 
 /* Validates the requests and enqueues them on `stream` (no graph, no autotuning: the configuration
  * cached for the workload key is used when there is one, else a default): each LINEAR request
- * with at least 2^21 output pixels as a grid of its own (the per-call kernel), the others as ONE persistent launch, its descriptors staged in stream-ordered device memory. The request
- * structs may be freed on return; the device buffers must stay valid until the launches complete.
+ * with at least 2^21 output pixels as a grid of its own (the per-call kernel), the others as ONE persistent
+ * launch, its descriptors staged in stream-ordered device memory. The request structs may be freed on return; the device buffers must stay valid until the launches complete.
  * Results are bit-identical to nb_extract_central_slices_3d on each request. */
 NB_API int nb_extract_batch_launch(int32_t remap, const nb_extract_request_ex* requests, int64_t n_requests,
                                    const nb_options* options, void* stream);

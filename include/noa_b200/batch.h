@@ -56,7 +56,7 @@ enum { NB_BATCH_AUTOTUNE = 1, NB_BATCH_PERSISTENT_ONLY = 2 };
  * so it writes the outputs) and captures the launch into a CUDA graph. Synchronizes `stream`.
  * LINEAR batches over complex volumes (no input weights or w-window) hold a pair copy (16 bytes per
  * rfft voxel, rows and planes padded by a few elements) of each volume whose requests read at least two
- * output pixels per voxel of it (three of a volume of 2^24 voxels and more, for requests run as grids); the
+ * output pixels per voxel of it and 3 * 2^17 in all (three of a volume of 2^24 voxels and more, for requests run as grids); the
  * graph rebuilds these copies at every run, so changes to the volumes between runs are seen. A LINEAR request with at least 2^16 output pixels runs,
  * in the graph, as a grid of its own (the per-call kernel) on a parallel branch, from its volume or, once
  * it is written, from its volume's copy; the copies are made meanwhile on a higher-priority branch

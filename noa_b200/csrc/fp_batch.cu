@@ -450,7 +450,9 @@ namespace {
 // 202 and 1168 us without and 25, 107 and 808 us with copies; over 384^3 as grids of their own 767 and 759 us, 60 requests of
 // 3.2 there 1155 and 1063 us. (The persistent kernel gains from about one pixel per voxel on, 23 and 21 us at 96^3, 115
 // and 70 us at 192^3; the line is at two for the memory that a batch holds and the time to make it.)
-constexpr int64_t BATCH_PAIRS = 2, BATCH_PAIRS_LARGE = 3;
+// Below BATCH_PAIRS_MIN pixels its launch costs more than it gives: 34 requests over 33^3 to 99^3, 2.3 pixels per voxel of
+// the smallest (40 k pixels), 35 us with its copy and 31 without.
+constexpr int64_t BATCH_PAIRS = 2, BATCH_PAIRS_LARGE = 3, BATCH_PAIRS_MIN = 3 * (int64_t(1) << 17);
 constexpr size_t NO_JOB = ~size_t(0);  // of a direct request that reads its volume, not a pair copy
 
 // Whether a request gets a grid of its own: LINEAR without a w-window and at least `least` output pixels.
@@ -693,8 +695,8 @@ void plan_pairs(nb_extract_batch_t* h, bool allow_direct) {
     }
     for (const Vol& v : vols) {
         const int64_t vox = static_cast<int64_t>(v.a->vol_d) * v.a->vol_h * (v.a->vol_w / 2 + 1);
-        if (v.pixels < (vox < (int64_t(1) << 24) ? BATCH_PAIRS : BATCH_PAIRS_LARGE) * vox &&
-            v.persistent < BATCH_PAIRS * vox)
+        if (v.pixels < BATCH_PAIRS_MIN || (v.pixels < (vox < (int64_t(1) << 24) ? BATCH_PAIRS : BATCH_PAIRS_LARGE) * vox &&
+                                           v.persistent < BATCH_PAIRS * vox))
             continue;
         ProjArgs copy = *v.a;
         pad_pairs(copy);

@@ -167,13 +167,14 @@ cudaError_t launch_linear(const ProjArgs& a, const float4* pairs, cudaStream_t s
 
 // Without a pair copy: whether the launch is large enough for four pixels per thread. One pixel per thread
 // (extract_kernel) has four times the threads to hide the taps' latency with, up to so many rounds of the chip's
-// 2048 threads per SM (303 k pixels): five for complex values, six with input weights, four for real values. us of
+// 2048 threads per SM (303 k pixels): three, two in a batch, whose grids fill the chip together. us of
 // extract_kernel and of extract_linear_kernel, means over boxes of 48 to 256: 0.65 M pixels 12.5 and 14.1, 1.3 M 21.9 and
 // 21.9, 1.8 M 28.8 and 27.5; with weights 1.3 M 31.3 and 33.5, 1.8 M 41.4 and 41.8; real 0.65 M 11.4 and 12.1, 0.9 M 14.8
-// and 15.2, 1.3 M 20.0 and 19.0.
-bool use_linear_kernel(const ProjArgs& a) {
+// and 15.2, 1.3 M 20.0 and 19.0. With a cutoff of 0.3 fewer taps are waited for: 1.1 M with weights 16.4 and 14.6. Batches
+// by lines at five, at two and at none: 59 requests of 0.02 M to 1.2 M 352, 329 and 309, 41 of 0.06 M to 2.1 M 322, 291 and 276,
+// but 49 of up to 0.2 M 48 at two and 57 at none, 29 of 30 k 27 and 33.
+bool use_linear_kernel(const ProjArgs& a, int rounds) {
     const int64_t pixels = a.n_slices * a.slice_h * static_cast<int64_t>(a.slice_w / 2 + 1);
-    const int rounds = !a.in_cplx ? 4 : a.in_w.present && a.out_w.present ? 6 : 5;
     return a.interp == I_LINEAR && a.wsize <= 1 && pixels >= static_cast<int64_t>(sm_count()) * 2048 * rounds;
 }
 
@@ -353,14 +354,14 @@ extract_window_kernel(const __grid_constant__ ProjArgs a, int ntx) {
 }
 
 template<int I, bool IN_C, bool OUT_C>
-cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
+cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream, int rounds) {
     const int wp = a.slice_w / 2 + 1;
     const int ntx = (wp + TX - 1) / TX, nty = (a.slice_h + TY - 1) / TY;
     if (a.n_slices == 0)
         return cudaSuccess;
     const dim3 grid(static_cast<unsigned>(ntx * nty), static_cast<unsigned>(a.n_slices < 65535 ? a.n_slices : 65535));
     if constexpr (I == I_LINEAR) {
-        if (use_linear_kernel(a))
+        if (use_linear_kernel(a, rounds))
             return a.wide_in ? launch_linear<false, IN_C, OUT_C, int64_t>(a, nullptr, stream)
                              : launch_linear<false, IN_C, OUT_C, int32_t>(a, nullptr, stream);
     }
@@ -379,12 +380,12 @@ cudaError_t launch_typed(const ProjArgs& a, cudaStream_t stream) {
 }
 
 template<int I>
-cudaError_t launch_interp(const ProjArgs& a, cudaStream_t stream) {
+cudaError_t launch_interp(const ProjArgs& a, cudaStream_t stream, int rounds = 3) {
     if (a.in_cplx && a.out_cplx)
-        return launch_typed<I, true, true>(a, stream);
+        return launch_typed<I, true, true>(a, stream, rounds);
     if (a.in_cplx)
-        return launch_typed<I, true, false>(a, stream);
-    return launch_typed<I, false, false>(a, stream);
+        return launch_typed<I, true, false>(a, stream, rounds);
+    return launch_typed<I, false, false>(a, stream, rounds);
 }
 
 } // namespace
@@ -428,7 +429,7 @@ cudaError_t launch_make_pairs(const ProjArgs& a, float4* pairs, cudaStream_t str
     return cudaLaunchKernelEx(&cfg, make_pairs<int64_t>, a, pairs);
 }
 
-cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream) { return launch_interp<I_LINEAR>(a, stream); }
+cudaError_t launch_extract_volume(const ProjArgs& a, cudaStream_t stream) { return launch_interp<I_LINEAR>(a, stream, 2); }
 
 cudaError_t launch_extract(const ProjArgs& a, cudaStream_t stream) {
     if (a.n_slices > 0 && use_pairs(a, stream)) {

@@ -190,16 +190,17 @@ inline bool pairs_apply(const ProjArgs& a) {
 }
 
 // From how many output pixels on a LINEAR extraction is faster through a pair copy made for it: two per
-// voxel, four where the copy is twice the L2 and more (2^24 voxels), and 3 * 2^19 for its allocation and launch;
+// voxel, four where the copy is twice the L2 and more (2^24 voxels), and 2^21 for its allocation and launch;
 // 3 * 2^17 in a stream capture, where the allocation is a node of the graph. Called one after another, us without and
 // with: 64^3 x 384 slices (6 pixels per voxel) 18 and 19, x 512 (8) 21 and 20; 96^3 x 192 (2) 21 and 21, x 384 (4) 31 and 29;
 // 128^3 x 192 (1.5) 28 and 27, x 256 (2) 33 and 31, x 512 (4) 57 and 48; 160^3 x 320 (2) 58 and 51; 256^3 x 512 (2) 196 and 187,
 // x 768 (3) 276 and 243; 384^3 x 1152 (3) 959 and 962, x 1536 (4) 1328 and 1253; 512^3 x 1536 (3) 2489 and 2622, x 2048 (4) 3349 and
 // 3390, x 4096 (8) 6778 and 6473. In a graph: 64^3 x 160 (2.5) 9.1 and 9.1, x 192 (3) 10.6 and 9.0; 96^3 x 192 (2) 19 and 16;
-// 128^3 x 256 (2) 32 and 26; 384^3 x 960 (2.5) 812 and 823.
+// 128^3 x 256 (2) 32 and 26; 384^3 x 960 (2.5) 812 and 823. A smaller cutoff leaves less to gain: 77^3 x 575 slices (1.7 M
+// pixels) with a cutoff of 0.3 25 and 29.
 inline bool pairs_pay(int64_t pixels, int64_t voxels, cudaStream_t stream) {
     return pixels >= (voxels < (int64_t(1) << 24) ? 2 : 4) * voxels && pixels >= 3 * (int64_t(1) << 17) &&
-           (pixels >= 3 * (int64_t(1) << 19) || stream_capturing(stream));
+           (pixels >= int64_t(1) << 21 || stream_capturing(stream));
 }
 
 // The same of the w-windowed extraction, by samples: three per voxel (four), and 2 M.

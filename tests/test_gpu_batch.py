@@ -214,12 +214,12 @@ def test_linear_batch_pair_copies_follow_volume_updates(tmp_path, monkeypatch):
 
 @pytest.mark.parametrize("persistent_only", [False, True])
 def test_linear_batch_copies_from_two_pixels_per_voxel(persistent_only):
-    """A batch holds a copy of every volume that its requests read two pixels per voxel of, however few they
-    are and whichever kernel they run in; the same bits as the per-call entry point."""
+    """A batch holds a copy of every volume that its requests read two pixels per voxel of, and 3 * 2^17 pixels,
+    whichever kernel they run in; the same bits as the per-call entry point."""
     import torch
     from noa_b200.batch import ExtractBatch
-    reqs, _ = _large_requests([(48, 60), (64, 100), (48, 40), (40, 79), (64, 30), (96, 193)], seed=15)
-    assert _copies(reqs, persistent_only=persistent_only) == 3  # 48 (100 slices), 64 (130) and 96; not 40 (79)
+    reqs, _ = _large_requests([(48, 300), (64, 150), (48, 40), (40, 79), (64, 45), (96, 193), (32, 600), (100, 150)], seed=15)
+    assert _copies(reqs, persistent_only=persistent_only) == 3  # 48 (340 slices), 64 (195) and 96; 32 has too few pixels, 100 too few per voxel, 40 both
     batch = ExtractBatch("hc2h", reqs, interp="linear", autotune=False, persistent_only=persistent_only)
     assert (batch.info()["n_direct"] > 0) != persistent_only
     batch.run()

@@ -194,7 +194,7 @@ def test_linear_extraction_groups(kw, copies, remap):
     _check(default_case("extract", remap=remap, seed=706, **kw), 1e-5, copies)
 
 
-# The rule on making a pair copy (two pixels per voxel, 3 * 2^19 pixels), its padded strides, and requests of a
+# The rule on making a pair copy (two pixels per voxel, 2^21 pixels), its padded strides, and requests of a
 # batch that read their volume in grids of their own: the same bits with and without the copy, in every layout
 # and with every form of the coordinates and outputs that a copy serves.
 def _with_and_without_pair_copy(n, size, count, remap="hc2h", form="plain"):

@@ -141,7 +141,7 @@ def test_gpu_constant_input_rasterize():
 @pytest.mark.parametrize("remap", ["h2h", "h2hc", "hc2h", "hc2hc"])
 @pytest.mark.parametrize("out_dt", ["c32", "f32"])
 def test_gpu_extract_pair_path(remap, out_dt):
-    """Enough slices that extraction takes the pair-copy fast path (at least 3 * 2^19 pixels, 2 per voxel)."""
+    """Enough slices that extraction takes the pair-copy fast path (at least 2^21 pixels, 2 per voxel)."""
     import gpu_run
     call = build(default_case("extract", remap=remap, n=32, nslices=3900, out_dt=out_dt, out_w=True, seed=640))
     ref = clone(call)

@@ -75,7 +75,9 @@ def test_concurrent_threads_match_sequential_calls():
     assert not errors, errors
     for (_, out, grid, grid_w), (r_out, r_grid, r_w) in zip(jobs, refs):
         assert torch.equal(out, r_out)
-        assert _rel(grid, 3 * r_grid) <= 1e-6 and _rel(grid_w, 3 * r_w) <= 1e-6
+        # The atomic sums' order differs. The voxels at the origin, which set the norm, sum about 3 terms of each of 3 x 130
+        # slices: a random walk of 1200 roundings of half an ulp, 2^-24 sqrt(1200) = 2.1e-6 of them; 1.05e-6 was seen.
+        assert _rel(grid, 3 * r_grid) <= 2.1e-6 and _rel(grid_w, 3 * r_w) <= 2.1e-6
 
 
 def test_errors_are_reported_per_thread():
